@@ -108,7 +108,8 @@ def draw(rng):
             break
     c = _search("", nchans, fhi, flo, tsamp, ndump, "\n".join(lines), precision=rng.choice(["fp32", "fp16", "bf16"]),
                 beams=rng.choice([1, 1, 2]), source=rng.choice(["device", "device", "host", "pinned", "float"]),
-                rfi=rng.random() < 0.5, iqr=rng.random() < 0.15, zapthre=rng.choice([0.0, 4.0]))
+                iqr=rng.random() < 0.15, zapthre=rng.choice([0.0, 4.0]))
+    c["rfi"] = flt == RFI and c["zapthre"] > 0 and c["source"] != "float"  # unfiltered RFI is all points, no search
     while not _modest(c):  # a shorter DM range, then fewer rows, until the case is no larger than the listed ones
         lines = c["plan"].split("\n")
         p = lines[-1].split()
