@@ -38,32 +38,124 @@ struct RpMeta {
     int levels; /* log2(nchans) */
     long soff;  /* first entry of its shift plan (levels x nchans) */
     long roff;  /* first entry of its row order hrange (nchans) */
+    long rowoff; /* first of its S/N-map rows among the batch's */
 };
 
 inline unsigned nblk(long n, int b) { return (unsigned)((n + b - 1) / b); }
 
-/* Candidate::zdot, first loop (candidate.cpp:837-859): per channel, double mean and (float
- * square) power, then x = (x - mean) / std in double, stored as float. */
-__global__ void k_rp_zdot_norm(float *__restrict__ buf, const RpMeta *__restrict__ m)
+/* ---- sequential per-row chains ----------------------------------------------------------- */
+/* The reference's statistics, running sums and kadane scans are chains: each sample's float or
+ * double operation needs the previous one's result, so a row is one lane's work.  What need
+ * not be serial is the memory side.  A warp takes 32 rows; RT-sample tiles of all 32 are
+ * copied into shared memory by cp.async, one coalesced 128-byte row piece per instruction,
+ * RNB - 1 tiles ahead of the scan, and each lane walks its own row of the tile (33-word pitch:
+ * no bank conflicts).  The chain then runs at its arithmetic latency; a lane reading its row
+ * straight from memory waited for an uncoalesced load at every sample (statistics of six
+ * candidates of 1024 channels x 6640 samples: 3.8 ms a launch before, 0.71 ms so; boxcar
+ * chains and search of 6 x 1024 rows of 1048 samples: 5.1 ms before, 0.61 + 0.23 ms). */
+constexpr int RT = 32;
+constexpr int RNB = 4;
+typedef float RpTile[RT][RT + 1];
+
+__device__ __forceinline__ void rp_cp4(float *dst, const float *src)
 {
-    const RpMeta c = m[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= c.nchan) return;
-    float *r = buf + c.off + (long)j * c.pitch;
-    double tmpmean = 0., tmpstd = 0.;
-    for (long i = 0; i < c.nbin; i++) {
-        tmpmean += r[i];
-        tmpstd += r[i] * r[i];
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void rp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void rp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(RNB - 2) : "memory"); }
+
+/* step(t, v) for t = 0 .. cnt-1 on every lane, v[k] = sample (start[k] + t) mod n of the lane's
+ * row (start[k] + cnt <= 2n + 1); rows 0..nrow-1 at `rows` with `pitch`.  The lanes of a warp
+ * call it together with the same cnt, n and nrow; lanes at or past nrow see undefined values.
+ * tile: K * RNB tiles of the warp. */
+template <int K, typename Step>
+__device__ __forceinline__ void rp_scan(RpTile *tile, const float *rows, long pitch, int nrow, long n,
+                                        const long (&start)[K], long cnt, Step step)
+{
+    const int lane = threadIdx.x & 31;
+    const long ntl = (cnt + RT - 1) / RT;
+    auto stage = [&](long tl) {
+        if (tl < ntl) {
+            const long t = tl * RT + lane;
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                RpTile &tb = tile[k * RNB + (int)(tl % RNB)];
+#pragma unroll 4
+                for (int r = 0; r < nrow; r++) {
+                    long i = __shfl_sync(0xffffffffu, start[k], r) + t;
+                    i = i >= n ? i - n : i;
+                    i = i >= n ? i - n : i;
+                    if (t < cnt) rp_cp4(&tb[r][lane], rows + r * pitch + i);
+                }
+            }
+        }
+        rp_commit(); /* one group per tile, empty past the end */
+    };
+    __syncwarp(); /* the previous scan's tiles are read no more */
+#pragma unroll
+    for (int b = 0; b < RNB - 1; b++) stage(b);
+    for (long tl = 0; tl < ntl; tl++) {
+        rp_wait();
+        __syncwarp(); /* every lane's copies of tile tl are there; tile tl-1 is read no more */
+        const long t0 = tl * RT;
+        const int b = (int)(tl % RNB);
+        float v[K];
+        if (t0 + RT <= cnt) {
+#pragma unroll 8
+            for (int q = 0; q < RT; q++) {
+#pragma unroll
+                for (int k = 0; k < K; k++) v[k] = tile[k * RNB + b][lane][q];
+                step(t0 + q, v);
+            }
+        } else {
+            for (int q = 0; q < (int)(cnt - t0); q++) {
+#pragma unroll
+                for (int k = 0; k < K; k++) v[k] = tile[k * RNB + b][lane][q];
+                step(t0 + q, v);
+            }
+        }
+        stage(tl + RNB - 1);
     }
+}
+
+/* Candidate::zdot, first loop (candidate.cpp:837-859): per channel, double mean and (float
+ * square) power; std 1 where it is 0. */
+__global__ void __launch_bounds__(32) k_rp_zdot_sums(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                     double *__restrict__ mean, double *__restrict__ std)
+{
+    __shared__ RpTile tile[RNB];
+    const RpMeta c = m[blockIdx.y];
+    const int j0 = blockIdx.x * 32, j = j0 + threadIdx.x;
+    if (j0 >= c.nchan) return;
+    double tmpmean = 0., tmpstd = 0.;
+    rp_scan<1>(tile, buf + c.off + (long)j0 * c.pitch, c.pitch, min(32, c.nchan - j0), c.nbin, {0}, c.nbin,
+               [&](long, const float(&v)[1]) {
+                   tmpmean += v[0];
+                   tmpstd += v[0] * v[0];
+               });
+    if (j >= c.nchan) return;
     tmpmean /= c.nbin;
     tmpstd /= c.nbin;
     tmpstd -= tmpmean * tmpmean;
     tmpstd = sqrt(tmpstd);
     if (tmpstd == 0.) tmpstd = 1.;
-    for (long i = 0; i < c.nbin; i++) {
-        r[i] = (float)(r[i] - tmpmean);
-        r[i] = (float)(r[i] / tmpstd);
-    }
+    mean[c.coff + j] = tmpmean;
+    std[c.coff + j] = tmpstd;
+}
+
+/* its second half, one CTA per channel: x = (x - mean) / std in double, stored as float after
+ * each step */
+__global__ void __launch_bounds__(256) k_rp_zdot_norm(float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                      const double *__restrict__ mean, const double *__restrict__ std)
+{
+    const RpMeta c = m[blockIdx.y];
+    const int j = blockIdx.x;
+    if (j >= c.nchan) return;
+    float *r = buf + c.off + (long)j * c.pitch;
+    const double mu = mean[c.coff + j], sd = std[c.coff + j];
+    for (long i = threadIdx.x; i < c.nbin; i += blockDim.x) r[i] = (float)((float)(r[i] - mu) / sd);
 }
 
 /* zdot's zero-DM series: s[i] = sum over channels in order (double), / nchan (:857-864) */
@@ -73,145 +165,192 @@ __global__ void k_rp_zdot_s(const float *__restrict__ buf, const RpMeta *__restr
     const RpMeta c = m[blockIdx.y];
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nbin) return;
+    const float *p = buf + c.off + i;
     double acc = 0.;
-    for (int j = 0; j < c.nchan; j++) acc += buf[c.off + (long)j * c.pitch + i];
+    int j = 0;
+    for (; j + 16 <= c.nchan; j += 16) { /* sixteen loads in flight, added in channel order */
+        float v[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) v[r] = p[(long)(j + r) * c.pitch];
+#pragma unroll
+        for (int r = 0; r < 16; r++) acc += v[r];
+    }
+    for (; j < c.nchan; j++) acc += p[(long)j * c.pitch];
     acc /= c.nchan;
     s[blockIdx.y * soff_stride + i] = acc;
 }
 
-/* zdot's least-squares fit and subtraction (:866-895) */
-__global__ void k_rp_zdot_fit(float *__restrict__ buf, const RpMeta *__restrict__ m,
-                              const double *__restrict__ s_all, long soff_stride)
+/* zdot's least-squares fit (:866-885): the sums over each channel (xe, xs), and by the last CTA
+ * of a candidate those of s (se, ss), which are the same for every channel */
+__global__ void __launch_bounds__(32) k_rp_zdot_fit(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                    const double *__restrict__ s_all, long soff_stride,
+                                                    double *__restrict__ xe_all, double *__restrict__ xs_all,
+                                                    double2 *__restrict__ ses)
+{
+    __shared__ RpTile tile[RNB];
+    const RpMeta c = m[blockIdx.y];
+    const double *s = s_all + blockIdx.y * soff_stride;
+    if (blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x == 0) {
+            double se = 0., ss = 0.;
+#pragma unroll 16
+            for (long i = 0; i < c.nbin; i++) {
+                const double v = s[i];
+                se += v;
+                ss += v * v;
+            }
+            ses[blockIdx.y] = make_double2(se, ss);
+        }
+        return;
+    }
+    const int j0 = blockIdx.x * 32, j = j0 + threadIdx.x;
+    if (j0 >= c.nchan) return;
+    double xe = 0., xs = 0.;
+    rp_scan<1>(tile, buf + c.off + (long)j0 * c.pitch, c.pitch, min(32, c.nchan - j0), c.nbin, {0}, c.nbin,
+               [&](long i, const float(&v)[1]) {
+                   xe += v[0];
+                   xs += v[0] * s[i];
+               });
+    if (j >= c.nchan) return;
+    xe_all[c.coff + j] = xe;
+    xs_all[c.coff + j] = xs;
+}
+
+/* the fit's coefficients and its subtraction (:880-895), one CTA per channel */
+__global__ void __launch_bounds__(256) k_rp_zdot_sub(float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                     const double *__restrict__ s_all, long soff_stride,
+                                                     const double *__restrict__ xe_all,
+                                                     const double *__restrict__ xs_all,
+                                                     const double2 *__restrict__ ses)
 {
     const RpMeta c = m[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.x;
     if (j >= c.nchan) return;
     float *r = buf + c.off + (long)j * c.pitch;
     const double *s = s_all + blockIdx.y * soff_stride;
-    double xe = 0., xs = 0., se = 0., ss = 0., alpha = 0., beta = 0.;
-    for (long i = 0; i < c.nbin; i++) {
-        xe += r[i];
-        xs += r[i] * s[i];
-        se += s[i];
-        ss += s[i] * s[i];
-    }
+    const double xe = xe_all[c.coff + j], xs = xs_all[c.coff + j], se = ses[blockIdx.y].x, ss = ses[blockIdx.y].y;
+    double alpha = 0., beta = 0.;
     const double tmp = se * se - ss * c.nbin;
     if (tmp != 0) {
         alpha = (xe * se - xs * c.nbin) / tmp;
         beta = (xs * se - xe * ss) / tmp;
     }
-    for (long i = 0; i < c.nbin; i++) r[i] = (float)(r[i] - (alpha * s[i] + beta));
+    for (long i = threadIdx.x; i < c.nbin; i += blockDim.x) r[i] = (float)(r[i] - (alpha * s[i] + beta));
 }
 
 /* Candidate::get_stats (:429-534) for one polarisation: the half-length window of least sum
- * (circular), mean/var of the data over it in double, and skewness, kurtosis and lag-1
- * autocorrelation in float. */
-__global__ void k_rp_stats(const float *__restrict__ buf, const RpMeta *__restrict__ m,
-                           double *__restrict__ mean, double *__restrict__ var, float *__restrict__ skew,
-                           float *__restrict__ kurt, float *__restrict__ ac)
+ * (circular), then over that window either skewness, kurtosis and lag-1 autocorrelation in
+ * float (SHAPE, what azap reads) or mean and variance in double (what normalize reads). */
+template <bool SHAPE>
+__global__ void __launch_bounds__(32) k_rp_stats(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                 double *__restrict__ mean, double *__restrict__ var,
+                                                 float *__restrict__ skew, float *__restrict__ kurt,
+                                                 float *__restrict__ ac)
 {
+    __shared__ RpTile tile[2 * RNB];
     const RpMeta c = m[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= c.nchan) return;
-    const float *r = buf + c.off + (long)j * c.pitch;
+    const int j0 = blockIdx.x * 32, j = j0 + threadIdx.x;
+    if (j0 >= c.nchan) return;
+    const float *rows = buf + c.off + (long)j0 * c.pitch;
+    const int nrow = min(32, c.nchan - j0);
     const long nbin = c.nbin, h = nbin / 2;
-    auto sumif = [&](long i) { return 0.f + r[i]; }; /* data_sumif starts at 0 and adds the data */
+    /* data_sumif starts at 0 and adds the data: 0.f + x */
     float boxsum = 0.;
-    for (long i = 0; i < h; i++) boxsum += sumif(i);
+    rp_scan<1>(tile, rows, c.pitch, nrow, nbin, {0}, h, [&](long, const float(&v)[1]) { boxsum += 0.f + v[0]; });
     float mn = boxsum;
-    long istart = 0, iend = h;
-    for (long i = 0; i < nbin; i++) {
-        boxsum -= sumif(i);
-        boxsum += sumif((i + h) % nbin);
+    int istart = 0;
+    rp_scan<2>(tile, rows, c.pitch, nrow, nbin, {0, h}, nbin, [&](long i, const float(&v)[2]) {
+        boxsum -= 0.f + v[0];
+        boxsum += 0.f + v[1];
         if (boxsum < mn) {
             mn = boxsum;
-            istart = i + 1;
-            iend = h + i + 1;
+            istart = (int)i + 1;
+        }
+    });
+    const long q = c.coff + j;
+    if (SHAPE) {
+        const float tmp_mean = mn / h;
+        float tmp_var = 0., sk = 0., ku = 0., a1 = 0., last = 0;
+        rp_scan<1>(tile, rows, c.pitch, nrow, nbin, {(long)istart}, h, [&](long, const float(&v)[1]) {
+            const float t = (0.f + v[0]) - tmp_mean;
+            const float t2 = t * t, t3 = t2 * t, t4 = t3 * t;
+            tmp_var += t2;
+            sk += t3;
+            ku += t4;
+            a1 += t * last;
+            last = t;
+        });
+        tmp_var /= h;
+        if (tmp_var <= 0) {
+            sk = 0.;
+            ku = 0.;
+            a1 = 0.;
+        }
+        sk /= h;
+        sk /= tmp_var * sqrtf(tmp_var);
+        ku /= h;
+        ku /= tmp_var * tmp_var;
+        ku -= 3.;
+        a1 /= h - 1;
+        a1 /= tmp_var;
+        if (j < c.nchan) {
+            skew[q] = sk;
+            kurt[q] = ku;
+            ac[q] = a1;
+        }
+    } else {
+        double mu = 0., v2 = 0.;
+        rp_scan<1>(tile, rows, c.pitch, nrow, nbin, {(long)istart}, h, [&](long, const float(&v)[1]) {
+            mu += v[0];
+            v2 += v[0] * v[0];
+        });
+        mu /= h;
+        v2 /= h;
+        v2 -= mu * mu;
+        if (j < c.nchan) {
+            mean[q] = mu;
+            var[q] = v2;
         }
     }
-    double mu = 0., v = 0.;
-    for (long i = istart; i < iend; i++) {
-        mu += r[i % nbin];
-        v += r[i % nbin] * r[i % nbin];
-    }
-    mu /= h;
-    v /= h;
-    v -= mu * mu;
-    const float tmp_mean = mn / h;
-    float tmp_var = 0., sk = 0., ku = 0., a1 = 0., last = 0;
-    for (long i = istart; i < iend; i++) {
-        const float t = sumif(i % nbin) - tmp_mean;
-        const float t2 = t * t, t3 = t2 * t, t4 = t3 * t;
-        tmp_var += t2;
-        sk += t3;
-        ku += t4;
-        a1 += t * last;
-        last = t;
-    }
-    tmp_var /= h;
-    if (tmp_var <= 0) {
-        sk = 0.;
-        ku = 0.;
-        a1 = 0.;
-    }
-    sk /= h;
-    sk /= tmp_var * sqrtf(tmp_var);
-    ku /= h;
-    ku /= tmp_var * tmp_var;
-    ku -= 3.;
-    a1 /= h - 1;
-    a1 /= tmp_var;
-    const long q = c.coff + j;
-    mean[q] = mu;
-    var[q] = v;
-    skew[q] = sk;
-    kurt[q] = ku;
-    ac[q] = a1;
 }
 
-/* Candidate::dedisperse, incoherent branch (:106-140): row j rotated left by its delay */
-__global__ void k_rp_dedisp(const float *__restrict__ src, float *__restrict__ dst,
-                            const RpMeta *__restrict__ m, const int *__restrict__ delay)
+/* Candidate::dedisperse, incoherent branch (:106-140): row j rotated left by its delay; the
+ * first keep[candidate] samples, all that the chop which follows leaves.  One CTA per channel. */
+__global__ void __launch_bounds__(256) k_rp_dedisp(const float *__restrict__ src, float *__restrict__ dst,
+                                                   const RpMeta *__restrict__ m, const int *__restrict__ delay,
+                                                   const long *__restrict__ keep)
 {
     const RpMeta c = m[blockIdx.y];
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)c.nchan * c.nbin) return;
-    const int j = (int)(e / c.nbin);
-    const long i = e - (long)j * c.nbin;
-    const long d = delay[c.coff + j];
-    const long k = i + d < c.nbin ? i + d : i + d - c.nbin;
-    dst[c.off + (long)j * c.pitch + i] = src[c.off + (long)j * c.pitch + k];
+    const int j = blockIdx.x;
+    if (j >= c.nchan) return;
+    const long o = c.off + (long)j * c.pitch, d = delay[c.coff + j], n = keep[blockIdx.y];
+    for (long i = threadIdx.x; i < n; i += blockDim.x) dst[o + i] = src[o + (i + d < c.nbin ? i + d : i + d - c.nbin)];
 }
 
-/* data *= weights[j] (azap :610-621, zap :641-653) */
-__global__ void k_rp_scale(float *__restrict__ buf, const RpMeta *__restrict__ m,
-                           const float *__restrict__ w)
+/* data *= weights[j] (azap :610-621, zap :641-653), one CTA per channel */
+__global__ void __launch_bounds__(256) k_rp_scale(float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                  const float *__restrict__ w)
 {
     const RpMeta c = m[blockIdx.y];
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)c.nchan * c.nbin) return;
-    const int j = (int)(e / c.nbin);
-    float *p = buf + c.off + (long)j * c.pitch + (e - (long)j * c.nbin);
-    *p *= w[c.coff + j];
+    const int j = blockIdx.x;
+    if (j >= c.nchan) return;
+    float *r = buf + c.off + (long)j * c.pitch;
+    const float f = w[c.coff + j];
+    for (long i = threadIdx.x; i < c.nbin; i += blockDim.x) r[i] *= f;
 }
 
-/* Candidate::normalize (:536-567) */
-__global__ void k_rp_normalize(float *__restrict__ buf, const RpMeta *__restrict__ m,
-                               const double *__restrict__ mean, const double *__restrict__ var)
+/* Candidate::normalize (:536-567), one CTA per channel */
+__global__ void __launch_bounds__(256) k_rp_normalize(float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                      const double *__restrict__ mean,
+                                                      const double *__restrict__ var)
 {
     const RpMeta c = m[blockIdx.y];
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)c.nchan * c.nbin) return;
-    const int j = (int)(e / c.nbin);
-    float *p = buf + c.off + (long)j * c.pitch + (e - (long)j * c.nbin);
+    const int j = blockIdx.x;
+    if (j >= c.nchan) return;
+    float *r = buf + c.off + (long)j * c.pitch;
     const double mu = mean[c.coff + j], v = var[c.coff + j];
-    if (v <= 0.) {
-        *p = (float)(*p - mu);
-    } else {
-        const float sd = (float)sqrt(v);
-        *p = (float)(*p - mu);
-        *p = *p / sd;
-    }
+    const float sd = v <= 0. ? 1.f : (float)sqrt(v); /* x / 1 is x */
+    for (long i = threadIdx.x; i < c.nbin; i += blockDim.x) r[i] = (float)(r[i] - mu) / sd;
 }
 
 /* Candidate::clip (:656-708): td x fd sums (fd outer, td inner) above thre zero their cells */
@@ -231,61 +370,76 @@ __global__ void k_rp_clip(float *__restrict__ buf, const RpMeta *__restrict__ m,
             for (int n = 0; n < td; n++) buf[c.off + (j * fd + k) * c.pitch + i * td + n] = 0.;
 }
 
-/* kadane<float> of the XLibs helpers as the reference tree's callers use it: a new maximum
- * needs a strictly larger sum, the running sum restarts after it drops below zero */
-__device__ float rp_kadane(const float *a, long n, long *start, long *end)
-{
-    float best = -INFINITY, cur = 0;
-    long cs = 0;
-    *start = 0;
-    *end = -1;
-    for (long i = 0; i < n; i++) {
-        cur = cur + a[i];
-        if (cur > best) {
-            best = cur;
-            *start = cs;
-            *end = i;
-        }
-        if (cur < 0) {
-            cur = 0;
-            cs = i + 1;
-        }
-    }
-    return best;
-}
-
-/* Candidate::kadaneF (:710-829), one thread per downsampled channel; ds: scratch of
- * stride `dstride` floats per (candidate, channel) */
-__global__ void k_rp_kadane(float *__restrict__ buf, const RpMeta *__restrict__ m, int td, int fd,
-                            float threshold, int nwidth, const float *__restrict__ width,
-                            const double *__restrict__ tbin, float *__restrict__ ds, long dstride)
+/* Candidate::kadaneF (:710-829): the td x fd sums (fd outer, td inner), one CTA per downsampled
+ * channel; ds: scratch rows of stride `dstride` per channel */
+__global__ void __launch_bounds__(128) k_rp_kadane_ds(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                      int td, int fd, float *__restrict__ ds, long dstride)
 {
     const RpMeta c = m[blockIdx.y];
     const long nsds = c.nbin / td, ncds = c.nchan / fd;
-    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long j = blockIdx.x;
     if (j >= ncds) return;
-    float *ch = ds + (c.coff + j) * dstride;
-    for (long i = 0; i < nsds; i++) ch[i] = 0.;
-    for (int k = 0; k < fd; k++)
-        for (int n = 0; n < td; n++)
-            for (long i = 0; i < nsds; i++) ch[i] += buf[c.off + (j * fd + k) * c.pitch + i * td + n];
-    const int wnlimit = (int)(nwidth * width[blockIdx.y] / tbin[blockIdx.y] / td);
-    const float var = (float)(td * fd);
-    for (int p = 0; p < 2; p++) {
-        if (p == 1)
-            for (long i = 0; i < nsds; i++) ch[i] = -ch[i];
-        long start, end;
-        const float boxsum = rp_kadane(ch, nsds, &start, &end);
-        const long wn = end - start + 1;
-        float snr2 = 0.;
-        if (wn > wnlimit) snr2 = boxsum * boxsum / (wn * var);
-        start *= td;
-        end += 1;
-        end *= td;
-        if (snr2 > threshold * threshold)
-            for (int k = 0; k < fd; k++)
-                for (long i = start; i < end; i++) buf[c.off + (j * fd + k) * c.pitch + i] = 0.;
+    for (long i = threadIdx.x; i < nsds; i += blockDim.x) {
+        float acc = 0.;
+        for (int k = 0; k < fd; k++)
+            for (int n = 0; n < td; n++) acc += buf[c.off + (j * fd + k) * c.pitch + i * td + n];
+        ds[(c.coff + j) * dstride + i] = acc;
     }
+}
+
+/* kadane<float> of the XLibs helpers as the reference tree's callers use it (a new maximum
+ * needs a strictly larger sum, the running sum restarts after it drops below zero), on the
+ * positive (z = 0) or the negated (z = 1) sums, then the S/N test with no minimum window
+ * (replot_fil passes nwidth 0): ranges[4*channel + 2*z] = first and last-plus-one sample, -1
+ * where nothing is zapped */
+__global__ void __launch_bounds__(32) k_rp_kadane_scan(const float *__restrict__ ds, const RpMeta *__restrict__ m,
+                                                       int td, int fd, float threshold, long dstride,
+                                                       long *__restrict__ ranges)
+{
+    __shared__ RpTile tile[RNB];
+    const RpMeta c = m[blockIdx.y];
+    const long nsds = c.nbin / td, ncds = c.nchan / fd;
+    const long j0 = (long)blockIdx.x * 32, j = j0 + threadIdx.x;
+    if (j0 >= ncds) return;
+    const bool neg = blockIdx.z;
+    float best = -INFINITY, cur = 0;
+    int cs = 0, start = 0, end = -1;
+    rp_scan<1>(tile, ds + (c.coff + j0) * dstride, dstride, (int)min(32L, ncds - j0), max(nsds, 1L), {0}, nsds,
+               [&](long i, const float(&v)[1]) {
+                   cur = cur + (neg ? -v[0] : v[0]);
+                   if (cur > best) {
+                       best = cur;
+                       start = cs;
+                       end = (int)i;
+                   }
+                   if (cur < 0) {
+                       cur = 0;
+                       cs = (int)i + 1;
+                   }
+               });
+    if (j >= ncds) return;
+    const float var = (float)(td * fd);
+    const long wn = (long)end - start + 1;
+    float snr2 = 0.;
+    if (wn > 0) snr2 = best * best / (wn * var);
+    const bool zap = snr2 > threshold * threshold;
+    long *o = ranges + 4 * (c.coff + j) + 2 * blockIdx.z;
+    o[0] = zap ? (long)start * td : -1;
+    o[1] = zap ? (long)(end + 1) * td : -1;
+}
+
+/* its zapping, one CTA per channel */
+__global__ void __launch_bounds__(128) k_rp_kadane_apply(float *__restrict__ buf, const RpMeta *__restrict__ m, int fd,
+                                                         const long *__restrict__ ranges)
+{
+    const RpMeta c = m[blockIdx.y];
+    const int j = blockIdx.x;
+    if (j >= c.nchan / fd * fd) return;
+    const long *o = ranges + 4 * (c.coff + j / fd);
+    float *r = buf + c.off + (long)j * c.pitch;
+    for (int p = 0; p < 2; p++)
+        if (o[2 * p] >= 0)
+            for (long i = o[2 * p] + threadIdx.x; i < o[2 * p + 1]; i += blockDim.x) r[i] = 0.;
 }
 
 /* Candidate::downsample(1, fd) (:381-427): channel sums in order, out of place */
@@ -302,57 +456,44 @@ __global__ void k_rp_fsum(const float *__restrict__ src, float *__restrict__ dst
     dst[c.off + j * c.pitch + i] = acc;
 }
 
-/* Candidate::optimize (:899-966): the Hough input rows, frequency-descending, zero padded to
- * nchans rows */
-__global__ void k_rp_hough_fill(const float *__restrict__ buf, float *__restrict__ h,
-                                const RpMeta *__restrict__ m, const int *__restrict__ flip)
+/* One level of the transform of hough_transform.h:29-55 (depth = levels-1-t), one CTA per output
+ * row: for block irow of 2*nrowsub rows, row k of the first half becomes x0 + rot(y, d0) and row
+ * k of the second half x0 + rot(y, d1), y being the old second-half row and
+ * rot(y, d)[i] = y[(i+d) mod ncol].  The first level reads Candidate::optimize's input
+ * (:899-966): the channels, frequency-descending, rows past them zero.  A candidate's last
+ * level writes the transform's output order, row hrange[r]; later levels of a batch whose
+ * other candidates have more rows copy it. */
+__global__ void __launch_bounds__(256) k_rp_hough_level(const float *__restrict__ buf, const float *__restrict__ hin,
+                                                        float *__restrict__ hout, const RpMeta *__restrict__ m,
+                                                        const int *__restrict__ shift,
+                                                        const int *__restrict__ hrange,
+                                                        const int *__restrict__ flip, int t)
 {
     const RpMeta c = m[blockIdx.y];
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)c.nchans * c.nbin) return;
-    const long j = e / c.nbin, i = e - j * c.nbin;
-    float v = 0.;
-    if (j < c.nchan) {
-        const long src = flip[blockIdx.y] ? c.nchan - 1 - j : j;
-        v = 0.f + buf[c.off + src * c.pitch + i];
-    }
-    h[c.hoff + e] = v;
-}
-
-/* One level of the transform of hough_transform.h:29-55 (depth = levels-1-t): for block irow of
- * 2*nrowsub rows, row k of the first half becomes x0 + rot(y, d0) and row k of the second half
- * x0 + rot(y, d1), y being the old second-half row and rot(y, d)[i] = y[(i+d) mod ncol]. */
-__global__ void k_rp_hough_level(const float *__restrict__ hin, float *__restrict__ hout,
-                                 const RpMeta *__restrict__ m, const int *__restrict__ shift, int t)
-{
-    const RpMeta c = m[blockIdx.y];
-    const long ncol = c.nbin;
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)c.nchans * ncol) return;
-    const long r = e / ncol, i = e - r * ncol;
-    const int depth = c.levels - 1 - t;
-    if (depth < 0) {
-        hout[c.hoff + e] = hin[c.hoff + e];
+    const long ncol = c.nbin, r = blockIdx.x;
+    if (r >= c.nchans) return;
+    if (t >= c.levels) {
+        for (long i = threadIdx.x; i < ncol; i += blockDim.x)
+            hout[c.hoff + r * ncol + i] = hin[c.hoff + r * ncol + i];
         return;
     }
-    const long nrowsub = (long)c.nchans >> (depth + 1);
+    const long nrowsub = 1L << t;
     const long blk = r / (2 * nrowsub), k = r - blk * 2 * nrowsub;
-    const int *sh = shift + c.soff + (long)(c.levels - 1 - depth) * c.nchans;
-    const long d = sh[blk * 2 * nrowsub + k];
+    const long d = shift[c.soff + (long)t * c.nchans + blk * 2 * nrowsub + k];
     const long x0 = k < nrowsub ? r : r - nrowsub, y = x0 + nrowsub;
-    const long iy = i + d < ncol ? i + d : i + d - ncol;
-    hout[c.hoff + e] = hin[c.hoff + x0 * ncol + i] + hin[c.hoff + y * ncol + iy];
-}
-
-/* the transform's last step: output row hrange[j] = row j */
-__global__ void k_rp_hough_perm(const float *__restrict__ hin, float *__restrict__ hout,
-                                const RpMeta *__restrict__ m, const int *__restrict__ hrange)
-{
-    const RpMeta c = m[blockIdx.y];
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)c.nchans * c.nbin) return;
-    const long j = e / c.nbin, i = e - j * c.nbin;
-    hout[c.hoff + (long)hrange[c.roff + j] * c.nbin + i] = hin[c.hoff + e];
+    const bool fl = flip[blockIdx.y];
+    auto row = [&](long j) -> const float * {
+        if (t > 0) return hin + c.hoff + j * ncol;
+        return j < c.nchan ? buf + c.off + (fl ? c.nchan - 1 - j : j) * c.pitch : nullptr;
+    };
+    const float *xr = row(x0), *yr = row(y);
+    float *o = hout + c.hoff + (t == c.levels - 1 ? (long)hrange[c.roff + r] : r) * ncol;
+    for (long i = threadIdx.x; i < ncol; i += blockDim.x) {
+        const long iy = i + d < ncol ? i + d : i + d - ncol;
+        const float a = xr ? xr[i] : 0.f, b = yr ? yr[iy] : 0.f;
+        /* the input rows are 0 + data */
+        o[i] = t > 0 ? a + b : (0.f + a) + (0.f + b);
+    }
 }
 
 /* peak_search's profile (:1115-1129): sum of the channels in order, from 0 */
@@ -362,104 +503,158 @@ __global__ void k_rp_profile(const float *__restrict__ buf, float *__restrict__ 
     const RpMeta c = m[blockIdx.y];
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nbin) return;
+    const float *p = buf + c.off + i;
     float acc = 0.;
-    for (int j = 0; j < c.nchan; j++) acc += buf[c.off + (long)j * c.pitch + i];
+    int j = 0;
+    for (; j + 16 <= c.nchan; j += 16) { /* sixteen loads in flight, added in channel order */
+        float v[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) v[r] = p[(long)(j + r) * c.pitch];
+#pragma unroll
+        for (int r = 0; r < 16; r++) acc += v[r];
+    }
+    for (; j < c.nchan; j++) acc += p[(long)j * c.pitch];
     h[c.hoff + i] = acc;
 }
 
-/* matched_filter / peak_search boxcar of one row (:1000-1063, :1131-1180): double mean and
- * variance (get_mean_var), float circular running sum of (x - mean) in double, widths of the
- * float ladder, S >= best keeps the later width.  csum: scratch of 2*nbin floats per row. */
-__global__ void k_rp_boxcar(const float *__restrict__ h, const RpMeta *__restrict__ m,
-                            const int *__restrict__ rows, const float *__restrict__ vwn,
-                            const int *__restrict__ nbox, long wstride, float *__restrict__ snr,
-                            int *__restrict__ wid, float *__restrict__ csump)
+/* The chains of matched_filter / peak_search (:1000-1030, :1131-1150): per row the double mean
+ * and variance (get_mean_var), then twice round the row the float running sum of (x - mean),
+ * each addition in double.  csum: 2*nbin floats per row, written through a shared-memory tile. */
+__global__ void __launch_bounds__(32) k_rp_csum(const float *__restrict__ h, const RpMeta *__restrict__ m,
+                                                const int *__restrict__ rows, double *__restrict__ var_all,
+                                                float *__restrict__ csump)
 {
+    __shared__ RpTile tile[RNB];
+    __shared__ RpTile outt;
     const RpMeta c = m[blockIdx.y];
-    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= rows[blockIdx.y]) return;
+    const int lane = threadIdx.x;
+    const long j0 = (long)blockIdx.x * 32, j = j0 + lane;
+    if (j0 >= rows[blockIdx.y]) return;
     const long nbin = c.nbin;
-    const float *tim = h + c.hoff + j * nbin;
-    float *cs = csump + (c.hoff + j * nbin) * 2;
-    float *vS = snr + c.hoff + j * nbin;
-    int *vw = wid + c.hoff + j * nbin;
+    const int nrow = (int)min(32L, rows[blockIdx.y] - j0);
+    const float *tim = h + c.hoff + j0 * nbin;
+    float *cs = csump + (c.hoff + j0 * nbin) * 2;
     double s1 = 0., s2 = 0.;
-    for (long i = 0; i < nbin; i++) {
-        const double v = tim[i];
+    rp_scan<1>(tile, tim, nbin, nrow, nbin, {0}, nbin, [&](long, const float(&x)[1]) {
+        const double v = x[0];
         s1 += v;
         s2 += v * v;
-    }
+    });
     const double mean = s1 / nbin, var = s2 / nbin - mean * mean;
+    if (lane < nrow) var_all[c.rowoff + j] = var;
     float csum = 0.;
-    for (long i = 0; i < nbin; i++) {
-        csum += tim[i] - mean;
-        cs[i] = csum;
-    }
-    for (long i = nbin; i < 2 * nbin; i++) {
-        csum += tim[i - nbin] - mean;
-        cs[i] = csum;
-    }
-    for (long i = 0; i < nbin; i++) {
-        vS[i] = 0.;
-        vw[i] = 0;
-    }
-    if (var > 0) {
-        const float *lad = vwn + blockIdx.y * wstride;
-        for (int k = 0; k < nbox[blockIdx.y]; k++) {
-            const int wn = (int)lad[k];
-            const int wl = wn / 2 + 1, wh = (wn - 1) / 2;
-            const float temp = (float)sqrt(1. / (wn * var));
-            for (long i = wl; i < nbin; i++) {
-                const float S = (cs[i + wh] - cs[i - wl]) * temp;
-                if (S >= vS[i]) {
-                    vS[i] = S;
-                    vw[i] = wn;
-                }
-            }
-            for (long i = nbin; i < nbin + wl; i++) {
-                const float S = (cs[i + wh] - cs[i - wl]) * temp;
-                if (S >= vS[i - nbin]) {
-                    vS[i - nbin] = S;
-                    vw[i - nbin] = wn;
-                }
-            }
+    rp_scan<1>(tile, tim, nbin, nrow, nbin, {0}, 2 * nbin, [&](long i, const float(&x)[1]) {
+        csum += x[0] - mean;
+        const int q = (int)(i % RT);
+        outt[lane][q] = csum;
+        if (q == RT - 1 || i == 2 * nbin - 1) {
+            __syncwarp();
+            if (lane <= q)
+#pragma unroll 4
+                for (int r = 0; r < nrow; r++) cs[r * 2 * nbin + i - q + lane] = outt[r][lane];
+            __syncwarp();
         }
+    });
+}
+
+/* best of a row or candidate: the first largest S in row-major order (the scan of :1065-1078) */
+struct RpBest {
+    long idx;
+    float S;
+    int wn;
+};
+__device__ __forceinline__ bool rp_before(float S, long i, float T, long k) { return S > T || (S == T && i < k); }
+
+/* The boxcar search of one row (:1031-1063, :1151-1180), one CTA per row: S over the float
+ * ladder from the circular running sum, S >= best keeps the later width.  Widths in chunks of
+ * RP_W, their factors computed once per CTA; a sample's best lives in the map between chunks. */
+constexpr int RP_W = 128;
+
+__global__ void __launch_bounds__(256) k_rp_match(const RpMeta *__restrict__ m, const int *__restrict__ rows,
+                                                  const float *__restrict__ vwn, const int *__restrict__ nbox,
+                                                  long wstride, const double *__restrict__ var_all,
+                                                  const float *__restrict__ csump, float *__restrict__ snr,
+                                                  int *__restrict__ wid, RpBest *__restrict__ rbest)
+{
+    __shared__ float temp[RP_W];
+    __shared__ int wns[RP_W];
+    __shared__ RpBest red[8];
+    const RpMeta c = m[blockIdx.y];
+    const long j = blockIdx.x;
+    if (j >= rows[blockIdx.y]) return;
+    const long nbin = c.nbin;
+    const float *cs = csump + (c.hoff + j * nbin) * 2;
+    float *vS = snr + c.hoff + j * nbin;
+    int *vw = wid + c.hoff + j * nbin;
+    const double var = var_all[c.rowoff + j];
+    const int nw = var > 0 ? nbox[blockIdx.y] : 0;
+    const float *lad = vwn + blockIdx.y * wstride;
+    RpBest mine{0x7fffffffffffffffL, -1.f, 0};
+    for (int w0 = 0; w0 == 0 || w0 < nw; w0 += RP_W) {
+        const int nc = min(RP_W, nw - w0);
+        __syncthreads();
+        for (int w = threadIdx.x; w < nc; w += blockDim.x) {
+            const int wn = (int)lad[w0 + w];
+            wns[w] = wn;
+            temp[w] = (float)sqrt(1. / (wn * var));
+        }
+        __syncthreads();
+        for (long i = threadIdx.x; i < nbin; i += blockDim.x) {
+            float b = w0 ? vS[i] : 0.f;
+            int bw = w0 ? vw[i] : 0;
+#pragma unroll 4
+            for (int w = 0; w < nc; w++) {
+                const int wn = wns[w], wl = wn / 2 + 1, wh = (wn - 1) / 2;
+                const long k = i >= wl ? i : i + nbin;
+                const float S = (cs[k + wh] - cs[k - wl]) * temp[w];
+                if (S >= b) {
+                    b = S;
+                    bw = wn;
+                }
+            }
+            vS[i] = b;
+            vw[i] = bw;
+            if (w0 + RP_W >= nw && rp_before(b, i, mine.S, mine.idx)) mine = RpBest{i, b, bw};
+        }
+    }
+    /* the row's first largest S (never a NaN: a NaN score fails S >= best) */
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    for (int off = 16; off >= 1; off >>= 1) {
+        const RpBest o{__shfl_xor_sync(0xffffffffu, mine.idx, off), __shfl_xor_sync(0xffffffffu, mine.S, off),
+                       __shfl_xor_sync(0xffffffffu, mine.wn, off)};
+        if (rp_before(o.S, o.idx, mine.S, mine.idx)) mine = o;
+    }
+    if (lane == 0) red[wp] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 8; q++)
+            if (rp_before(red[q].S, red[q].idx, mine.S, mine.idx)) mine = red[q];
+        mine.idx += j * nbin;
+        rbest[c.rowoff + j] = mine;
     }
 }
 
-/* the first largest S of each candidate's map in row-major order (the scan of :1065-1078) */
-__global__ void __launch_bounds__(256) k_rp_argmax(const float *__restrict__ snr, const RpMeta *__restrict__ m,
-                                                   const int *__restrict__ rows, long *__restrict__ best)
+/* the candidate's best from its rows' */
+__global__ void __launch_bounds__(256) k_rp_best(const RpMeta *__restrict__ m, const int *__restrict__ rows,
+                                                 const RpBest *__restrict__ rbest, RpBest *__restrict__ best)
 {
+    __shared__ RpBest red[256];
     const RpMeta c = m[blockIdx.x];
-    const long n = (long)rows[blockIdx.x] * c.nbin;
-    const float *v = snr + c.hoff;
-    __shared__ float bv[256];
-    __shared__ long bi[256];
-    float b = -INFINITY;
-    long idx = -1;
-    for (long e = threadIdx.x; e < n; e += blockDim.x)
-        if (idx < 0 ? !(v[e] != v[e]) && v[e] >= b : v[e] > b) { /* NaN never wins */
-            b = v[e];
-            idx = e;
-        }
-    bv[threadIdx.x] = b;
-    bi[threadIdx.x] = idx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float B = -INFINITY;
-        long I = -1;
-        for (int t = 0; t < (int)blockDim.x; t++) {
-            if (bi[t] < 0) continue;
-            if (I < 0 || bv[t] > B || (bv[t] == B && bi[t] < I)) {
-                B = bv[t];
-                I = bi[t];
-            }
-        }
-        /* the reference starts from element 0: a NaN there, or no number at all, keeps it */
-        if (n > 0 && (v[0] != v[0] || I < 0 || !(B > v[0]))) I = 0;
-        best[blockIdx.x] = I;
+    RpBest mine{0x7fffffffffffffffL, -1.f, 0};
+    for (long j = threadIdx.x; j < rows[blockIdx.x]; j += blockDim.x) {
+        const RpBest o = rbest[c.rowoff + j];
+        if (rp_before(o.S, o.idx, mine.S, mine.idx)) mine = o;
     }
+    red[threadIdx.x] = mine;
+    __syncthreads();
+    for (int h = 128; h >= 1; h >>= 1) {
+        if (threadIdx.x < h) {
+            const RpBest o = red[threadIdx.x + h];
+            if (rp_before(o.S, o.idx, mine.S, mine.idx)) red[threadIdx.x] = mine = o;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) best[blockIdx.x] = mine;
 }
 
 } // namespace
@@ -479,7 +674,7 @@ struct RpHost {
     std::vector<double> f;
     /* Hough geometry (step 12) */
     int nchans = 1, levels = 0;
-    long hoff = 0, soff = 0, roff = 0, rows = 1;
+    long hoff = 0, soff = 0, roff = 0, rowoff = 0, rows = 1;
     double dms = 0., ddm = 0.;
 };
 
@@ -581,8 +776,8 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return set_cuda_error(cudaErrorNoDevice, "txg_replot", __FILE__, __LINE__);
 
     DevBuf mem;
-    float *buf[2] = {nullptr, nullptr}, *skew, *kurt, *ac, *w, *ds;
-    double *mean, *var, *zs;
+    float *buf[2] = {nullptr, nullptr}, *skew, *kurt, *ac, *w;
+    double *mean, *var;
     int *delay;
     RpMeta *dmeta;
     cudaStream_t st = nullptr;
@@ -606,8 +801,6 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
     RP_TRY(mem.alloc(&w, tchan));
     RP_TRY(mem.alloc(&delay, tchan));
     RP_TRY(mem.alloc(&dmeta, n));
-    RP_TRY(mem.alloc(&zs, (size_t)n * maxnbin));
-    RP_TRY(mem.alloc(&ds, (size_t)tchan * maxnbin));
     for (long b = 0; b < n; b++)
         RP_TRY(cudaMemcpyAsync(buf[0] + H[b].off, cands[b].data, sizeof(float) * H[b].nchan * H[b].nbin,
                                cudaMemcpyHostToDevice, st));
@@ -628,6 +821,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             m.levels = h.levels;
             m.soff = h.soff;
             m.roff = h.roff;
+            m.rowoff = h.rowoff;
         }
         return cudaMemcpyAsync(dmeta, meta.data(), sizeof(RpMeta) * n, cudaMemcpyHostToDevice, st);
     };
@@ -636,6 +830,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         for (auto &h : H) mc = std::max(mc, h.nchan);
         return mc;
     };
+    auto per32 = [&](int rows) { return nblk(rows, 32); }; /* warps of the row scans */
     auto maxelem = [&]() {
         long me = 0;
         for (auto &h : H) me = std::max(me, (long)h.nchan * h.nbin);
@@ -647,19 +842,45 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
 
     /* 1: zdot */
     if (o->zdot) {
-        k_rp_zdot_norm<<<dim3(nblk(maxchan(), 128), NB), 128, 0, st>>>(buf[cur], dmeta);
-        k_rp_zdot_s<<<dim3(nblk(maxnbin, 128), NB), 128, 0, st>>>(buf[cur], dmeta, zs, maxnbin);
-        k_rp_zdot_fit<<<dim3(nblk(maxchan(), 128), NB), 128, 0, st>>>(buf[cur], dmeta, zs, maxnbin);
+        double *zs, *xe, *xs;
+        double2 *ses;
+        RP_TRY(mem.alloc(&zs, (size_t)n * maxnbin));
+        RP_TRY(mem.alloc(&xe, tchan));
+        RP_TRY(mem.alloc(&xs, tchan));
+        RP_TRY(mem.alloc(&ses, n));
+        k_rp_zdot_sums<<<dim3(per32(maxchan()), NB), 32, 0, st>>>(buf[cur], dmeta, mean, var);
+        k_rp_zdot_norm<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
+        k_rp_zdot_s<<<dim3(nblk(maxnbin, 64), NB), 64, 0, st>>>(buf[cur], dmeta, zs, maxnbin);
+        k_rp_zdot_fit<<<dim3(per32(maxchan()) + 1, NB), 32, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
+        k_rp_zdot_sub<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
         RP_TRY(cudaGetLastError());
     }
     /* 2: get_stats (their skewness, kurtosis, autocorrelation drive azap) */
     std::vector<float> sk_h(tchan), ku_h(tchan), ac_h(tchan);
     if (upto >= 2) {
-        k_rp_stats<<<dim3(nblk(maxchan(), 128), NB), 128, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
+        k_rp_stats<true><<<dim3(per32(maxchan()), NB), 32, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
         RP_TRY(cudaGetLastError());
         RP_TRY(cudaMemcpyAsync(sk_h.data(), skew, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
         RP_TRY(cudaMemcpyAsync(ku_h.data(), kurt, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
         RP_TRY(cudaMemcpyAsync(ac_h.data(), ac, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
+    }
+    /* 4 (decided first, the rotation below then writes no more than it leaves):
+     * shrink_to_fit(2*nw, pow2bin, kadane td) (:234-264) */
+    std::vector<long> cut(n);
+    for (long b = 0; b < n; b++) {
+        const RpHost &h = H[b];
+        cut[b] = h.nbin;
+        if (upto < 4) continue;
+        const int nw2 = 2 * o->nwidth, factor = kad ? o->kadane[0] : 1;
+        long nbin_new = (long)(nw2 * h.width / h.tbin);
+        if (o->pow2bin) nbin_new = (long)std::pow(2, std::ceil(std::log2(nbin_new)));
+        nbin_new = (long)(std::ceil(nbin_new / factor) * factor);
+        if (nbin_new < h.nbin) cut[b] = nbin_new;
+        if (cut[b] < 4) {
+            cudaStreamSynchronize(st);
+            cudaStreamDestroy(st);
+            return set_arg_error("the chop to 2*nw*width leaves fewer than 4 samples");
+        }
     }
     /* 3: dedisperse at the candidate DM (incoherent) */
     if (upto >= 3) {
@@ -675,25 +896,16 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             }
         }
         RP_TRY(cudaMemcpyAsync(delay, dl.data(), sizeof(int) * tchan, cudaMemcpyHostToDevice, st));
-        k_rp_dedisp<<<dim3(nblk(maxelem(), 256), NB), 256, 0, st>>>(buf[cur], buf[cur ^ 1], dmeta, delay);
+        long *dcut;
+        RP_TRY(mem.alloc(&dcut, n));
+        RP_TRY(cudaMemcpyAsync(dcut, cut.data(), sizeof(long) * n, cudaMemcpyHostToDevice, st));
+        k_rp_dedisp<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], buf[cur ^ 1], dmeta, delay, dcut);
         RP_TRY(cudaGetLastError());
         RP_TRY(cudaStreamSynchronize(st)); /* dl goes out of scope */
         cur ^= 1;
     }
-    /* 4: shrink_to_fit(2*nw, pow2bin, kadane td) (:234-264) */
     if (upto >= 4) {
-        const int nw2 = 2 * o->nwidth, factor = kad ? o->kadane[0] : 1;
-        for (auto &h : H) {
-            long nbin_new = (long)(nw2 * h.width / h.tbin);
-            if (o->pow2bin) nbin_new = (long)std::pow(2, std::ceil(std::log2(nbin_new)));
-            nbin_new = (long)(std::ceil(nbin_new / factor) * factor);
-            if (nbin_new < h.nbin) h.nbin = nbin_new;
-        }
-        for (auto &h : H)
-            if (h.nbin < 4) {
-                cudaStreamDestroy(st);
-                return set_arg_error("the chop to 2*nw*width leaves fewer than 4 samples");
-            }
+        for (long b = 0; b < n; b++) H[b].nbin = cut[b];
         RP_TRY(push_meta());
     }
     /* 5: azap(zapthre) with the statistics of step 2 */
@@ -714,7 +926,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             }
         }
         RP_TRY(cudaMemcpyAsync(w, w_h.data(), sizeof(float) * tchan, cudaMemcpyHostToDevice, st));
-        k_rp_scale<<<dim3(nblk(maxelem(), 256), NB), 256, 0, st>>>(buf[cur], dmeta, w);
+        k_rp_scale<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, w);
         RP_TRY(cudaGetLastError());
     }
     /* 6: zap(zaplist): weights keep azap's zeros */
@@ -725,14 +937,14 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
                 for (int z = 0; z < o->nzap; z++)
                     if (h.f[j] >= o->zap[z][0] && h.f[j] <= o->zap[z][1]) w_h[h.coff + j] = 0;
         RP_TRY(cudaMemcpyAsync(w, w_h.data(), sizeof(float) * tchan, cudaMemcpyHostToDevice, st));
-        k_rp_scale<<<dim3(nblk(maxelem(), 256), NB), 256, 0, st>>>(buf[cur], dmeta, w);
+        k_rp_scale<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, w);
         RP_TRY(cudaGetLastError());
     }
     /* 7, 8: get_stats, normalize */
     if (upto >= 7)
-        k_rp_stats<<<dim3(nblk(maxchan(), 128), NB), 128, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
+        k_rp_stats<false><<<dim3(per32(maxchan()), NB), 32, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
     if (upto >= 8)
-        k_rp_normalize<<<dim3(nblk(maxelem(), 256), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
+        k_rp_normalize<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
     RP_TRY(cudaGetLastError());
     /* 9: clip */
     if (upto >= 9 && clp) {
@@ -743,22 +955,23 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
     }
     /* 10: kadaneF (nwidth 0, as replot_fil calls it) */
     if (upto >= 10 && kad) {
-        std::vector<float> wid_h(n);
-        std::vector<double> tb_h(n);
-        for (long b = 0; b < n; b++) {
-            wid_h[b] = H[b].width;
-            tb_h[b] = H[b].tbin;
+        const int td = o->kadane[0], fd = o->kadane[1];
+        long dstride = 1, ncmax = 0;
+        for (auto &h : H) {
+            dstride = std::max(dstride, h.nbin / td);
+            ncmax = std::max(ncmax, (long)h.nchan / fd);
         }
-        float *dwid;
-        double *dtb;
-        RP_TRY(mem.alloc(&dwid, n));
-        RP_TRY(mem.alloc(&dtb, n));
-        RP_TRY(cudaMemcpyAsync(dwid, wid_h.data(), sizeof(float) * n, cudaMemcpyHostToDevice, st));
-        RP_TRY(cudaMemcpyAsync(dtb, tb_h.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
-        k_rp_kadane<<<dim3(nblk(maxchan(), 64), NB), 64, 0, st>>>(buf[cur], dmeta, o->kadane[0], o->kadane[1],
-                                                                 (float)o->kadane[2], 0, dwid, dtb, ds, maxnbin);
-        RP_TRY(cudaGetLastError());
-        RP_TRY(cudaStreamSynchronize(st));
+        if (ncmax > 0) {
+            float *ds;
+            long *rng;
+            RP_TRY(mem.alloc(&ds, (size_t)tchan * dstride));
+            RP_TRY(mem.alloc(&rng, (size_t)tchan * 4));
+            k_rp_kadane_ds<<<dim3(ncmax, NB), 128, 0, st>>>(buf[cur], dmeta, td, fd, ds, dstride);
+            k_rp_kadane_scan<<<dim3(per32((int)ncmax), NB, 2), 32, 0, st>>>(ds, dmeta, td, fd, (float)o->kadane[2],
+                                                                          dstride, rng);
+            k_rp_kadane_apply<<<dim3(maxchan(), NB), 128, 0, st>>>(buf[cur], dmeta, fd, rng);
+            RP_TRY(cudaGetLastError());
+        }
     }
     /* 11: downsample(1, fd) */
     if (upto >= 11 && o->fd > 1) {
@@ -778,8 +991,8 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(push_meta());
     }
     /* 12: optimize + matched_filter, or peak_search */
-    std::vector<long> best(n, 0);
-    long hsize = 0;
+    std::vector<RpBest> best(n);
+    long hsize = 0, nrows = 0;
     std::vector<int> rows_h(n, 1);
     float *hb[2] = {nullptr, nullptr}, *dsnr = nullptr, *csump = nullptr, *dvwn = nullptr;
     int *dwidm = nullptr, *drows = nullptr, *dnbox = nullptr;
@@ -828,6 +1041,8 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
                 h.ddm = 0.;
             }
             rows_h[b] = (int)h.rows;
+            h.rowoff = nrows;
+            nrows += h.rows;
             hsize += h.rows * h.nbin;
         }
         int *dshift, *dhr, *dflip;
@@ -848,20 +1063,15 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(cudaMemcpyAsync(dflip, flip.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
         RP_TRY(cudaMemcpyAsync(drows, rows_h.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
         int hc = 0; /* which of hb holds the rows the boxcar reads */
-        long maxrows_elem = 0;
         int maxlevels = 0;
-        for (auto &h : H) {
-            maxrows_elem = std::max(maxrows_elem, h.rows * h.nbin);
-            maxlevels = std::max(maxlevels, h.levels);
-        }
+        for (auto &h : H) maxlevels = std::max(maxlevels, h.levels);
+        const int maxrows = *std::max_element(rows_h.begin(), rows_h.end());
         if (!o->nopt) {
-            k_rp_hough_fill<<<dim3(nblk(maxrows_elem, 256), NB), 256, 0, st>>>(buf[cur], hb[0], dmeta, dflip);
             for (int t = 0; t < maxlevels; t++) {
-                k_rp_hough_level<<<dim3(nblk(maxrows_elem, 256), NB), 256, 0, st>>>(hb[hc], hb[hc ^ 1], dmeta, dshift, t);
+                k_rp_hough_level<<<dim3(maxrows, NB), 256, 0, st>>>(buf[cur], hb[hc], hb[hc ^ 1], dmeta, dshift, dhr,
+                                                                   dflip, t);
                 hc ^= 1;
             }
-            k_rp_hough_perm<<<dim3(nblk(maxrows_elem, 256), NB), 256, 0, st>>>(hb[hc], hb[hc ^ 1], dmeta, dhr);
-            hc ^= 1;
         } else {
             k_rp_profile<<<dim3(nblk(maxnbin, 128), NB), 128, 0, st>>>(buf[cur], hb[0], dmeta);
         }
@@ -892,24 +1102,23 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(mem.alloc(&dnbox, n));
         RP_TRY(cudaMemcpyAsync(dvwn, lad_h.data(), sizeof(float) * lad_h.size(), cudaMemcpyHostToDevice, st));
         RP_TRY(cudaMemcpyAsync(dnbox, nbox_h.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
-        int maxrows = *std::max_element(rows_h.begin(), rows_h.end());
-        k_rp_boxcar<<<dim3(nblk(maxrows, 64), NB), 64, 0, st>>>(hb[hc], dmeta, drows, dvwn, dnbox, wstride,
-                                                                dsnr, dwidm, csump);
-        long *dbest;
+        double *dvar;
+        RpBest *drbest, *dbest;
+        RP_TRY(mem.alloc(&dvar, nrows));
+        RP_TRY(mem.alloc(&drbest, nrows));
         RP_TRY(mem.alloc(&dbest, n));
-        k_rp_argmax<<<NB, 256, 0, st>>>(dsnr, dmeta, drows, dbest);
+        k_rp_csum<<<dim3(per32(maxrows), NB), 32, 0, st>>>(hb[hc], dmeta, drows, dvar, csump);
+        k_rp_match<<<dim3(maxrows, NB), 256, 0, st>>>(dmeta, drows, dvwn, dnbox, wstride, dvar, csump, dsnr, dwidm,
+                                                     drbest);
+        k_rp_best<<<NB, 256, 0, st>>>(dmeta, drows, drbest, dbest);
         RP_TRY(cudaGetLastError());
-        RP_TRY(cudaMemcpyAsync(best.data(), dbest, sizeof(long) * n, cudaMemcpyDeviceToHost, st));
+        RP_TRY(cudaMemcpyAsync(best.data(), dbest, sizeof(RpBest) * n, cudaMemcpyDeviceToHost, st));
         RP_TRY(cudaStreamSynchronize(st));
         for (long b = 0; b < n; b++) {
             const RpHost &h = H[b];
-            float S = 0.f;
-            int wn = 0;
-            RP_TRY(cudaMemcpy(&S, dsnr + h.hoff + best[b], sizeof(float), cudaMemcpyDeviceToHost));
-            RP_TRY(cudaMemcpy(&wn, dwidm + h.hoff + best[b], sizeof(int), cudaMemcpyDeviceToHost));
-            const long maxdmid = best[b] / h.nbin, maxtid = best[b] % h.nbin;
-            out[b].snr = S;
-            out[b].width = (float)(wn * h.tbin);
+            const long maxdmid = best[b].idx / h.nbin, maxtid = best[b].idx % h.nbin;
+            out[b].snr = best[b].S;
+            out[b].width = (float)(best[b].wn * h.tbin);
             out[b].dm_maxsnr = o->nopt ? h.dm : h.dms + maxdmid * h.ddm;
             out[b].maxtid = maxtid;
             out[b].ndm = (int)h.rows;
