@@ -220,6 +220,7 @@ static constexpr size_t FIFO_MAX = 256;
 
 struct RowDev {
     int32_t *sub_start = nullptr, *d1 = nullptr, *d2 = nullptr, *vwn = nullptr, *zap = nullptr;
+    Stage1TDev s1t;
 };
 
 /* Per-beam scratch of the skewness/kurtosis channel zap. */
@@ -626,7 +627,7 @@ int run_block(txg_handle *h, int beam, const uint8_t *raw, const float *rawf = n
         const long tbase = counter - P.N - P.maxd1;
         TXG_CUDA_TRY(cudaMemsetAsync(sl.dcount, 0, 2 * sizeof(int), rs));
         launch_stage1(xcur, P.ldh, P.H - P.maxd1, P.C, P.N, P.nsub, P.ng, D.sub_start, D.d1,
-                      P.maxd1, P.maxch, b.ring, P.R, pmod(tbase, P.R), h->prec, P.s1_var,
+                      P.maxd1, P.maxch, b.ring, P.R, pmod(tbase, P.R), h->prec, P.s1_var, D.s1t,
                       sl.dcount + 1, rs);
         TXG_CUDA_TRY(cudaGetLastError());
         if (timing) TXG_CUDA_TRY(cudaEventRecord(sl.ev[3], rs));
@@ -781,7 +782,7 @@ int autotune_row(txg_handle *h, int r)
             float ms = 0.f;
             rc = time_of([&] {
                 launch_stage1(b.xh[0], P.ldh, P.H - P.maxd1, P.C, P.N, P.nsub, P.ng, D.sub_start,
-                              D.d1, P.maxd1, P.maxch, b.ring, P.R, 0, h->prec, v, err + 1, h->st);
+                              D.d1, P.maxd1, P.maxch, b.ring, P.R, 0, h->prec, v, D.s1t, err + 1, h->st);
             }, ms);
             if (rc) break;
             if (best < 0.f || ms < best) {
@@ -960,6 +961,18 @@ int txg_create(const txg_plan *plan, txg_handle **out)
             (rc = upload(h, &D.d2, P.d2)) || (rc = upload(h, &D.vwn, P.vwn)) ||
             (rc = upload(h, &D.zap, P.zap_chan)))
             return bail(rc);
+        Stage1T t;
+        if (stage1t_tables(P.d1.data(), P.C, P.nsub, P.ng, P.sub_start.data(), P.maxch, t)) {
+            if ((rc = upload(h, &D.s1t.rel, t.rel)) || (rc = upload(h, &D.s1t.first, t.first)) ||
+                (rc = upload(h, &D.s1t.span, t.span)))
+                return bail(rc);
+            D.s1t.npass = t.npass;
+            D.s1t.qpt = t.qpt;
+            D.s1t.cw = t.cw;
+            D.s1t.nb = t.nb;
+            D.s1t.widest = t.widest;
+            /* pageable uploads have left their vectors when the call returns */
+        }
     }
     h->br.resize(plan->nbeams);
     h->prep.resize(plan->nbeams);

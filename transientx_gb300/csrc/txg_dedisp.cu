@@ -79,6 +79,11 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
+/* the same, 16 bytes (both addresses 16-byte aligned) */
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
@@ -343,6 +348,287 @@ k_stage1r(const float *__restrict__ xh, long ldh, long col0, int C, long N, int 
             }
         }
     }
+}
+
+/* ---- tensor memory as a file of shiftable windows ------------------------------------------ */
+/* A dedispersion sum reads one window at many offsets: each (channel, delay) pair adds the same
+ * samples, shifted.  Read from shared memory that is one 4-byte word per addition, or per
+ * distinct delay, and the 128 bytes a clock of that pipe bound the kernel at a quarter of the
+ * FP32 add rate.  Tensor memory gives each of an SM's four schedulers 128 bytes a clock of its
+ * own, and one tcgen05.ld.32x32b.x16 reads 16 consecutive columns from any start column into
+ * every lane's registers: with consecutive samples of a lane in consecutive columns, a shift
+ * by d samples is a start column d further on, costs one instruction for 512 samples and
+ * leaves them aligned for the packed add.  Measured on the GB300 with 16 warps per SM: 12.4
+ * clocks per x16 load and scheduler, load and eight packed adds together at 0.76 of the add
+ * rate (0.58 with the windows' filling beside them). */
+__device__ __forceinline__ void tm_alloc(uint32_t *slot, int cols) /* one warp */
+{
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)),
+                 "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+__device__ __forceinline__ void tm_free(uint32_t t, int cols) /* the same warp */
+{
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(t), "r"(cols));
+}
+__device__ __forceinline__ void tm_ld16(uint32_t (&r)[16], uint32_t t)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                 "%13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                   "=r"(r[15])
+                 : "r"(t)
+                 : "memory");
+}
+__device__ __forceinline__ void tm_st8(uint32_t t, const float (&v)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(t),
+                 "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+/* The 160 threads whose warps share a scheduler (and with it 32 lanes of tensor memory) meet:
+ * what any of them stored is there for the others' loads, and their loads are done. */
+__device__ __forceinline__ void tm_team_sync(int team)
+{
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.sync %0, 160;" ::"r"(team + 1) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+/* acc[q] += the pair of samples (2q, 2q + 1) of a loaded window */
+__device__ __forceinline__ void tm_acc(float2 (&acc)[8], const uint32_t (&r)[16])
+{
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        acc[q] = __fadd2_rn(acc[q], make_float2(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1])));
+}
+/* Sixteen consecutive samples to 64-byte (float) or 32-byte (16-bit) aligned memory. */
+__device__ __forceinline__ void store16(float *o, const float2 (&a)[8])
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        reinterpret_cast<float4 *>(o)[q] = make_float4(a[2 * q].x, a[2 * q].y, a[2 * q + 1].x, a[2 * q + 1].y);
+}
+__device__ __forceinline__ uint32_t pack2(float2 v, __half *)
+{
+    const __half2 h = __floats2half2_rn(v.x, v.y);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint32_t pack2(float2 v, __nv_bfloat16 *)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+template <typename T> __device__ __forceinline__ void store16(T *o, const float2 (&a)[8])
+{
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+        reinterpret_cast<uint4 *>(o)[q] = make_uint4(pack2(a[4 * q], o), pack2(a[4 * q + 1], o),
+                                                     pack2(a[4 * q + 2], o), pack2(a[4 * q + 3], o));
+}
+
+/* ---- stage 1 from tensor memory ----------------------------------------------------------- */
+/* CTA = (512-sample tile, subband).  Lane l of every warp owns samples 16l .. 16l+15 of the tile; a
+ * warp that adds has four consecutive coarse-DM groups (a quad), and the four such warps of a
+ * scheduler (a team) take consecutive quads.  The subband's channel windows are copied into
+ * shared memory once (one word of padding per 16, so that the lanes' starts fall in different
+ * banks) and stay while the teams walk all passes of up to 64 groups, each at its own pace.
+ * Per pass and block of `nb` channels the team's fifth warp, one block ahead, copies the piece
+ * of each channel that the team's quads need (16 samples and the spread of their delays) into
+ * the team's columns; the others add it at their groups' offsets.  A group with its
+ * neighbour's delay adds the values that are still in registers (two thirds of the steps
+ * between groups are 0 in the searches' plans).
+ *
+ * 1024 channels, 256 groups, 13156 samples, 16-bit subbands: 433 us with the best shared-memory
+ * shape below, 286 us so; 4096 channels and the searches' three rows, per row: 917 us and 785.
+ * Issue and latency bound it (2.1 of 4 instructions a clock, FP32 adds a third of them; 86
+ * registers leave five warps a scheduler).  Measured and not kept: the quads' common prefixes of
+ * equal delays summed once (a quarter fewer additions, but more branches and register moves:
+ * 346 us), one load per group without the branches (294 us), two loads in flight (293 us), loads
+ * one ahead (298 us), two groups a warp at eight warps a scheduler (342 us), the adding warps
+ * also filling (297 us). */
+constexpr int S1T_TT = 512;    /* samples per CTA */
+constexpr int S1T_THREADS = 640; /* 16 warps that add and 4 that fill */
+constexpr int S1T_COLS = 256;  /* columns of one of the two window buffers */
+constexpr int S1T_PASS = 64;   /* table entries (groups) per pass */
+/* words of a channel window beside its subband's largest delay: the tile and the rest of the
+ * last eight columns that a fill writes */
+constexpr int S1T_HALO = S1T_TT + 8;
+static_assert(S1T_TT == 32 * 16, "a lane holds 16 samples");
+
+/* rel: [channel][pass][64] column offsets from the set's window start; first: [channel][pass][4]
+ * that start, the delay of the set's first group rounded down to 8 (so that eight columns never
+ * straddle a padding word).  qpt: quads per team.  span: the largest delay of each subband. */
+template <typename T>
+__global__ void __launch_bounds__(S1T_THREADS, 1)
+k_stage1t(const float *__restrict__ xh, long ldh, long col0, int C, long N, int nsub, int ng,
+          const int32_t *__restrict__ sub_start, const uint16_t *__restrict__ rel,
+          const int32_t *__restrict__ first, int npass, int qpt, int cw, int nb,
+          const int32_t *__restrict__ span, int maxch, T *__restrict__ ring, long R, long tbase_mod)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ uint32_t tm_slot;
+    /* the shuffle tells the compiler that all of a warp has the same wp */
+    const int tid = threadIdx.x, lane = tid & 31, wp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int team = wp & 3, m = wp >> 2;
+    /* tables [channel][pass] x (64 offsets, 4 window starts), then the channel windows */
+    uint2 *rel_sm = reinterpret_cast<uint2 *>(smraw);
+    int32_t *first_sm = reinterpret_cast<int32_t *>(rel_sm + (size_t)maxch * npass * 16);
+    float *win = reinterpret_cast<float *>(first_sm + (size_t)maxch * npass * 4);
+    const int words = S1T_HALO + span[blockIdx.y], pitch = words + (words >> 4) + 1;
+    const int s = blockIdx.y, j0 = sub_start[s], jn = sub_start[s + 1] - j0;
+    /* tiles start where the ring index is a multiple of 16, so that a lane's samples are one
+     * aligned piece of the ring; samples before 0 are not stored */
+    const long u0 = (long)blockIdx.x * S1T_TT - (tbase_mod & 15);
+
+    if (wp == 0) tm_alloc(&tm_slot, 2 * S1T_COLS);
+    for (int e = tid; e < jn * npass * 8; e += S1T_THREADS) /* 16 bytes each */
+        cp_async16(rel_sm + 2 * e, rel + (size_t)j0 * npass * S1T_PASS + 8 * e);
+    for (int e = tid; e < jn * npass; e += S1T_THREADS)
+        cp_async16(first_sm + 4 * e, first + (size_t)j0 * npass * 4 + 4 * e);
+    for (int jj = wp; jj < jn; jj += S1T_THREADS / 32) {
+        float *d = win + (size_t)jj * pitch;
+        const float *x = xh + (long)(j0 + jj) * ldh;
+        const long c0 = u0 + col0; /* columns before the buffer hold no stored sample */
+        int n = lane;
+        for (; n < words && c0 + n < 0; n += 32) d[n + (n >> 4)] = 0.f;
+        x += c0;
+#pragma unroll 4
+        for (; n < words; n += 32) cp_async4(d + n + (n >> 4), x + n);
+    }
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tm = tm_slot + ((uint32_t)(32 * team) << 16);
+    const int nblk = (jn + nb - 1) / nb;
+    /* passes in which the team has groups; its steps are (pass, block of channels) */
+    int mypass = 0;
+    while (mypass < npass && (mypass * 4 + team) * qpt * 4 < ng) mypass++;
+    const int nstep = mypass * nblk;
+
+    if (m == 4) { /* the team's filling warp: the windows of a step's channels */
+        const float *lane_win = win + 17 * lane;
+        const int32_t *fp = first_sm + team;
+        /* the set's last group, the furthest, in the upper half */
+        const uint32_t *lp = reinterpret_cast<const uint32_t *>(rel_sm) + team * 8 + 2 * qpt - 1;
+        int n0 = *fp;
+        uint32_t last = *lp;
+        for (int i = 0, ps = 0, b = 0; i < nstep; i++) {
+            const int j1 = b * nb, je = min(jn, j1 + nb);
+            uint32_t t = tm + (i & 1) * S1T_COLS;
+            const float *row = lane_win + j1 * pitch;
+            b = b + 1 < nblk ? b + 1 : 0;
+            const int pn = b ? ps : ps + 1;
+            for (int jj = j1; jj < je; jj++, t += cw, row += pitch) {
+                /* 16 samples and the spread of the set's delays; n0 is a multiple of 8: a padding
+                 * word before every other eight */
+                const int wcols = 16 + (int)(last >> 16);
+                const float *x = row + n0 + (n0 >> 4), *y = x + (n0 >> 3 & 1), *z = x + 17;
+                float v[24];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[q] = x[q];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[8 + q] = y[8 + q];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[16 + q] = z[q];
+                const int odd = n0 & 8;
+                { /* the next channel's table entries */
+                    const int jx = jj + 1 < je ? jj + 1 : b * nb, px = jj + 1 < je ? ps : min(pn, npass - 1);
+                    n0 = fp[(jx * npass + px) * 4];
+                    last = lp[(jx * npass + px) * 32];
+                }
+                tm_st8(t, *reinterpret_cast<float(*)[8]>(v));
+                tm_st8(t + 8, *reinterpret_cast<float(*)[8]>(v + 8));
+                tm_st8(t + 16, *reinterpret_cast<float(*)[8]>(v + 16));
+                for (int c = 24; c < wcols; c += 8) {
+                    const float *w = x + c + ((odd + c) >> 4);
+                    float u[8];
+#pragma unroll
+                    for (int q = 0; q < 8; q++) u[q] = w[q];
+                    tm_st8(t + c, u);
+                }
+            }
+            ps = pn;
+            tm_wait_st();
+            tm_team_sync(team);
+        }
+    } else {
+        int i = 0;
+        for (int ps = 0; ps < mypass; ps++) {
+            const int quad = (ps * 4 + team) * qpt + m;
+            const bool mine = m < qpt && 4 * quad < ng;
+            float2 acc[4][8];
+#pragma unroll
+            for (int g = 0; g < 4; g++)
+#pragma unroll
+                for (int q = 0; q < 8; q++) acc[g][q] = make_float2(0.f, 0.f);
+            const uint2 *r = rel_sm + ps * 16 + team * 4 + m;
+            for (int j0b = 0; j0b < jn; j0b += nb) {
+                tm_team_sync(team); /* the block's windows are there, the other buffer is read no more */
+                uint32_t t = tm + (i++ & 1) * S1T_COLS;
+                const int n = min(nb, jn - j0b);
+                if (mine) {
+                    uint2 w = *r;
+                    w.x = __shfl_sync(0xffffffffu, w.x, 0);
+                    w.y = __shfl_sync(0xffffffffu, w.y, 0);
+#pragma unroll 1
+                    for (int k = 0; k < n; k++, t += cw) {
+                        const uint32_t c0 = w.x & 0xffffu, c1 = w.x >> 16, c2 = w.y & 0xffffu, c3 = w.y >> 16;
+                        r += npass * 16;
+                        if (k + 1 < n) w = *r;
+                        uint32_t v[16];
+                        tm_ld16(v, t + c0);
+                        w.x = __shfl_sync(0xffffffffu, w.x, 0);
+                        w.y = __shfl_sync(0xffffffffu, w.y, 0);
+                        tm_wait_ld();
+                        tm_acc(acc[0], v);
+                        if (c1 != c0) {
+                            tm_ld16(v, t + c1);
+                            tm_wait_ld();
+                        }
+                        tm_acc(acc[1], v);
+                        if (c2 != c1) {
+                            tm_ld16(v, t + c2);
+                            tm_wait_ld();
+                        }
+                        tm_acc(acc[2], v);
+                        if (c3 != c2) {
+                            tm_ld16(v, t + c3);
+                            tm_wait_ld();
+                        }
+                        tm_acc(acc[3], v);
+                    }
+                }
+            }
+            if (mine) {
+                const long u = u0 + 16 * lane;
+                long tr = tbase_mod + u;
+                tr = tr >= R ? tr - R : tr;
+                T *o = ring + ((size_t)(4 * quad) * nsub + s) * R + tr;
+                /* samples [lo, hi) of the sixteen are the block's */
+                const int lo = u < 0 ? (int)-u : 0, hi = u + 16 <= N ? 16 : (int)max(N - u, 0L);
+                const bool whole = lo == 0 && hi == 16;
+#pragma unroll
+                for (int g = 0; g < 4; g++, o += (size_t)nsub * R) {
+                    if (4 * quad + g >= ng) break;
+                    if (whole) {
+                        store16(o, acc[g]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 16; q++)
+                            if (q >= lo && q < hi) o[q] = to_store<T>((q & 1) ? acc[g][q / 2].y : acc[g][q / 2].x);
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (wp == 0) tm_free(tm_slot, 2 * S1T_COLS);
 }
 
 /* ---- 16-bit pairs ---------------------------------------------------------------------- */
@@ -648,6 +934,7 @@ inline unsigned nblk(long n, int b) { return (unsigned)((n + b - 1) / b); }
 
 constexpr size_t SMEM_BUDGET = 100 * 1024;     /* chunked stage 1: two CTAs per SM */
 constexpr size_t RESIDENT_BUDGET = 200 * 1024; /* whole-subband stage-1 windows */
+constexpr size_t S1T_SMEM = 224 * 1024;        /* k_stage1t: tables and windows */
 
 } // namespace
 
@@ -689,9 +976,67 @@ static void stage1_chunked(const float *xh, long ldh, long col0, int C, long N, 
                                                 wmax, ring, R, tbase_mod, err);
 }
 
+static size_t stage1t_smem(int maxch, int npass, int span)
+{
+    const long words = S1T_HALO + span, pitch = words + words / 16 + 1;
+    return (size_t)maxch * (npass * (S1T_PASS * sizeof(uint16_t) + 4 * sizeof(int32_t)) + pitch * sizeof(float));
+}
+
+/* The tables of k_stage1t for a row, or none (false) where it does not apply: tables and windows
+ * do not fit in shared memory, a team's groups spread over more than 112 samples in a channel, or
+ * delays do not grow with the group. */
+bool stage1t_tables(const int32_t *d1, int C, int nsub, int ng, const int32_t *sub_start, int maxch, Stage1T &t)
+{
+    t = Stage1T();
+    const int quads = (ng + 3) / 4, npass = (quads + 15) / 16, qpt = (quads + 4 * npass - 1) / (4 * npass);
+    t.span.assign(nsub, 0);
+    int widest = 0;
+    for (int s = 0; s < nsub; s++) {
+        for (int j = sub_start[s]; j < sub_start[s + 1]; j++)
+            t.span[s] = std::max(t.span[s], d1[(size_t)(ng - 1) * C + j]);
+        widest = std::max(widest, t.span[s]);
+    }
+    if (stage1t_smem(maxch, npass, widest) > S1T_SMEM) return false;
+    t.rel.assign((size_t)C * npass * S1T_PASS, 0);
+    t.first.assign((size_t)C * npass * 4, 0);
+    auto delay = [&](int g, int j) { return d1[(size_t)std::min(g, ng - 1) * C + j]; };
+    int spread = 0;
+    for (int j = 0; j < C; j++)
+        for (int set = 0; set < 4 * npass; set++) {
+            const int g0 = set * qpt * 4, d0 = delay(g0, j) & ~7;
+            t.first[(size_t)j * npass * 4 + set] = d0;
+            for (int k = 0, prev = d0; k < 4 * qpt; k++) {
+                const int d = delay(g0 + k, j);
+                if (d < prev) return false;
+                prev = d;
+                spread = std::max(spread, d - d0);
+                if (spread > 112) return false;
+                t.rel[((size_t)j * npass + set / 4) * S1T_PASS + (set % 4) * 16 + k] = (uint16_t)(d - d0);
+            }
+        }
+    t.npass = npass;
+    t.qpt = qpt;
+    t.cw = std::max((16 + spread + 7) / 8 * 8, 24); /* a fill writes 24 columns or more */
+    t.nb = S1T_COLS / t.cw;
+    t.widest = widest;
+    return true;
+}
+
+template <typename T>
+static void stage1t(const Stage1TDev &t, const float *xh, long ldh, long col0, int C, long N, int nsub, int ng,
+                    const int32_t *sub_start, int maxch, T *ring, long R, long tbase_mod, cudaStream_t st)
+{
+    const size_t smem = stage1t_smem(maxch, t.npass, t.widest);
+    auto kern = k_stage1t<T>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<dim3(nblk(N + (tbase_mod & 15), S1T_TT), nsub), S1T_THREADS, smem, st>>>(
+        xh, ldh, col0, C, N, nsub, ng, sub_start, t.rel, t.first, t.npass, t.qpt, t.cw, t.nb, t.span, maxch,
+        ring, R, tbase_mod);
+}
+
 /* Resident launch shapes (threads per set x samples per thread, thread sets x groups each),
  * the same for every ring precision:
- *   0 = 32x16 16x4 (default), 1 = 256x2 1x16, 2 = 512x1 1x16, 3 = 256x2 2x8, 4 = 256x2 2x16,
+ *   0 = from tensor memory (k_stage1t), where it does not apply 32x16 16x4 (18), 1 = 256x2 1x16, 2 = 512x1 1x16, 3 = 256x2 2x8, 4 = 256x2 2x16,
  *   5 = 256x1 2x8, 6 = 256x2 4x4, 7 = 128x4 4x8, 8 = 256x4 2x8, 9 = 128x4 2x8, 10 = 128x4 8x4,
  *   11 = 64x8 8x4, 12 = 64x8 4x4, 13 = 64x8 16x4, 14 = 64x8 8x8, 15 = 64x16 8x4,
  *   16 = 256x2 4x8, 17 = 32x8 16x8
@@ -707,9 +1052,13 @@ static void stage1_chunked(const float *xh, long ldh, long col0, int C, long N, 
 template <typename T>
 static void stage1_dispatch(const float *xh, long ldh, long col0, int C, long N,
                             int nsub, int ng, const int32_t *sub_start, const int32_t *d1, long maxd1,
-                            int maxch, T *ring, long R, long tbase_mod, int var, int *err,
+                            int maxch, T *ring, long R, long tbase_mod, int var, const Stage1TDev &t, int *err,
                             cudaStream_t st)
 {
+    if (var == 0 && t.npass > 0) {
+        stage1t<T>(t, xh, ldh, col0, C, N, nsub, ng, sub_start, maxch, ring, R, tbase_mod, st);
+        return;
+    }
     if (var < 0) { /* the chunked kernel, whatever fits */
         stage1_chunked<T>(xh, ldh, col0, C, N, nsub, ng, sub_start, d1, maxd1, maxch, ring, R, tbase_mod, err, st);
         return;
@@ -743,17 +1092,17 @@ static void stage1_dispatch(const float *xh, long ldh, long col0, int C, long N,
 
 void launch_stage1(const float *xh, long ldh, long col0, int C, long N, int nsub,
                    int ng, const int32_t *sub_start, const int32_t *d1, long maxd1, int maxch, void *ring,
-                   long R, long tbase_mod, int prec, int var, int *err, cudaStream_t st)
+                   long R, long tbase_mod, int prec, int var, const Stage1TDev &t, int *err, cudaStream_t st)
 {
     if (prec == TXG_PREC_BF16)
         stage1_dispatch<__nv_bfloat16>(xh, ldh, col0, C, N, nsub, ng, sub_start, d1, maxd1, maxch,
-                                       (__nv_bfloat16 *)ring, R, tbase_mod, var, err, st);
+                                       (__nv_bfloat16 *)ring, R, tbase_mod, var, t, err, st);
     else if (prec == TXG_PREC_FP16)
         stage1_dispatch<__half>(xh, ldh, col0, C, N, nsub, ng, sub_start, d1, maxd1, maxch,
-                                (__half *)ring, R, tbase_mod, var, err, st);
+                                (__half *)ring, R, tbase_mod, var, t, err, st);
     else
         stage1_dispatch<float>(xh, ldh, col0, C, N, nsub, ng, sub_start, d1, maxd1, maxch,
-                               (float *)ring, R, tbase_mod, var, err, st);
+                               (float *)ring, R, tbase_mod, var, t, err, st);
 }
 
 

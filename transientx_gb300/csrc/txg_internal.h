@@ -47,7 +47,7 @@ struct RowPlan {
     float kadT_thr = 0.f;      /* threKadaneT^2 */
     float mask_thr = 0.f;      /* threMask (IQR units) */
     /* dedispersion launch shapes */
-    int s1_var = 0;   /* resident stage-1 launch shape, 0 = default */
+    int s1_var = 0;   /* stage-1 launch shape, 0 = default */
     int s2_var = 0;   /* stage-2 threads per CTA, 0 = default (see txg_dedisp.cu) */
     int s2_kb = 0;    /* stage-2 shared memory per CTA, KB (0 = the kernel's default) */
 };
@@ -111,11 +111,25 @@ void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
 /* zp: C (mean, 1/sd) pairs of scratch */
 void launch_zdot(float *x, long ldx, int C, long N, float *s, double *sstats, float2 *zp,
                  cudaStream_t st);
+/* Delay tables of the stage-1 kernel that sums from tensor memory (txg_dedisp.cu) and the same
+ * on the device; npass 0 where that kernel does not apply to the row. */
+struct Stage1T {
+    std::vector<uint16_t> rel;
+    std::vector<int32_t> first, span;
+    int npass = 0, qpt = 0, cw = 0, nb = 0, widest = 0;
+};
+struct Stage1TDev {
+    uint16_t *rel = nullptr;
+    int32_t *first = nullptr, *span = nullptr;
+    int npass = 0, qpt = 0, cw = 0, nb = 0, widest = 0;
+};
+bool stage1t_tables(const int32_t *d1, int C, int nsub, int ng, const int32_t *sub_start, int maxch, Stage1T &t);
 /* Every precision reads the FP32 channel buffer and accumulates in FP32; the ring stores
  * FP32, BF16 or FP16 (prec).  var: resident launch shape (0 = default; see txg_dedisp.cu). */
 void launch_stage1(const float *xh, long ldh, long col0, int C, long N, int nsub,
                    int ng, const int32_t *sub_start, const int32_t *d1, long maxd1, int maxch,
-                   void *ring, long R, long tbase_mod, int prec, int var, int *err, cudaStream_t st);
+                   void *ring, long R, long tbase_mod, int prec, int var, const Stage1TDev &t, int *err,
+                   cudaStream_t st);
 long stage2_span(const int32_t *d2h, int nsub, int G, long ndm);
 long stage2_window(long span);
 /* s2_var: threads per CTA (0 = 32, 1 = 64, 2 = 128; 3-5 the same with half a group's DMs per
