@@ -217,6 +217,17 @@ def launches_per_block(sp, info, gated, precision="fp32"):
     return n
 
 
+def block_launches(sp, info, gated, precision="fp32"):
+    """launches_per_block less the downsample of the first filter where the equalize apply brings
+    it in its own pass (td 4, 8 or 16 and no zapped channels in between; txg_pre.cu k_ds)."""
+    n = launches_per_block(sp, info, gated, precision)
+    if sp.rfilist and not sp.zaplist and sp.rfilist[0][0] in ("kadaneF", "kadaneT", "mask"):
+        td, fd = int(sp.rfilist[0][1]), int(sp.rfilist[0][2])
+        if td in (4, 8, 16) and info.ndump >= td and info.nchans >= fd:
+            n -= 1
+    return n
+
+
 SKZAP_LAUNCHES = 3  # per block, all rows: moments, statistics, outlier selection
 
 
@@ -389,9 +400,9 @@ def run_single(args, wl):
                     stats["work"] += infos[r].ndm * infos[r].nsamples
                     stats["ncand"][r] += res.npoints
                     stats["gated"][r] += 1
-                    stats["launches"] += launches_per_block(wl.rows[r], infos[r], True, args.precision)
+                    stats["launches"] += block_launches(wl.rows[r], infos[r], True, args.precision)
                 else:
-                    stats["launches"] += launches_per_block(wl.rows[r], infos[r], False, args.precision)
+                    stats["launches"] += block_launches(wl.rows[r], infos[r], False, args.precision)
 
     def new_stats():
         return {"work": 0, "ncand": [0] * len(wl.rows), "gated": [0] * len(wl.rows),
@@ -689,7 +700,7 @@ class Lanes:
                         info = self.infos[C][r]
                         st["overflow"] += int(res.overflow)
                         st["d2h"] += 8 + 16 * res.npoints
-                        st["launches"] += launches_per_block(rows[r], info, bool(res.gated),
+                        st["launches"] += block_launches(rows[r], info, bool(res.gated),
                                                              self.precision)
                         if res.gated:
                             st["work"] += info.ndm * info.nsamples

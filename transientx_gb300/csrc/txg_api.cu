@@ -596,24 +596,28 @@ int run_block(txg_handle *h, int beam, const uint8_t *raw, const float *rawf = n
         if (P.bl_nw > 0) {
             launch_colmean(x, P.ldh, P.C, P.N, b.live, b.eqp, b.z, rs);
             launch_smooth(b.z, P.N, P.bl_nw, b.b, rs);
-            launch_eq_apply(x, P.ldh, P.C, P.N, b.eqp, b.b, b.live, rs);
-        } else {
-            launch_eq_apply(x, P.ldh, P.C, P.N, b.eqp, nullptr, b.live, rs);
         }
+        /* with nothing in between, the apply brings the first filter's downsampled block too */
+        const float *bl = P.bl_nw > 0 ? b.b : nullptr;
+        const int kind0 = P.cfg.nrfi > 0 && P.zap_chan.empty() ? P.cfg.rfi_kind[0] : 0;
+        const bool ds0 = (kind0 == TXG_RFI_KADANEF || kind0 == TXG_RFI_KADANET || kind0 == TXG_RFI_MASK) &&
+                         launch_eq_apply_ds(x, P.ldh, P.C, P.N, b.eqp, bl, b.live, P.cfg.rfi_td[0], P.cfg.rfi_fd[0],
+                                            b.ds, rs);
+        if (!ds0) launch_eq_apply(x, P.ldh, P.C, P.N, b.eqp, bl, b.live, rs);
         if (!P.zap_chan.empty())
             launch_zero_rows(x, P.ldh, D.zap, (int)P.zap_chan.size(), P.N, rs);
         for (int q = 0; q < P.cfg.nrfi; q++) {
             if (P.cfg.rfi_kind[q] == TXG_RFI_KADANEF)
                 launch_kadane(x, P.ldh, P.C, P.N, P.cfg.rfi_td[q], P.cfg.rfi_fd[q], P.kad_thr,
-                              P.kad_wnlimit[q], b.ds, b.ranges[q], rs);
+                              P.kad_wnlimit[q], b.ds, b.ranges[q], q == 0 && ds0, rs);
             else if (P.cfg.rfi_kind[q] == TXG_RFI_ZDOT)
                 launch_zdot(x, P.ldh, P.C, P.N, b.s, b.sst, b.zp, rs);
             else if (P.cfg.rfi_kind[q] == TXG_RFI_KADANET)
                 launch_kadaneT(x, P.ldh, P.C, P.N, P.cfg.rfi_td[q], P.cfg.rfi_fd[q], P.kadT_thr,
-                               P.kad_wnlimit[q], b.ds, b.ranges[q], rs);
+                               P.kad_wnlimit[q], b.ds, b.ranges[q], q == 0 && ds0, rs);
             else if (P.cfg.rfi_kind[q] == TXG_RFI_MASK)
                 launch_mask(x, P.ldh, P.C, P.N, P.cfg.rfi_td[q], P.cfg.rfi_fd[q], P.mask_thr, b.ds,
-                            b.sel, b.ranges[q], rs);
+                            b.sel, b.ranges[q], q == 0 && ds0, rs);
             else if (P.cfg.rfi_kind[q] == TXG_RFI_ZERO) {
                 /* zero-DM filter: the live-channel mean series off every live channel */
                 launch_colmean(x, P.ldh, P.C, P.N, b.live, nullptr, b.z, rs);

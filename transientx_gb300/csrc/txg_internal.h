@@ -88,6 +88,10 @@ void launch_eq_params_f32(const float *x, long ldx, int C, long N, float2 *eqp, 
 /* x <- standardised x, minus b on live channels when b is given */
 void launch_eq_apply(float *x, long ldx, int C, long N, const float2 *eqp, const float *b,
                      const uint8_t *live, cudaStream_t st);
+/* launch_eq_apply with b, and the td x fd downsample of the filter that follows in the same pass;
+ * false (nothing done) where it does not apply */
+bool launch_eq_apply_ds(float *x, long ldx, int C, long N, const float2 *eqp, const float *b, const uint8_t *live,
+                        int td, int fd, float *ds, cudaStream_t st);
 /* column mean (tp: of the standardised block, tp[j] = (mean, 1/sd) of channel j) */
 void launch_colmean(const float *x, long ldx, int C, long N, const uint8_t *live, const float2 *tp,
                     float *out, cudaStream_t st);
@@ -96,18 +100,19 @@ void launch_sub_series(float *x, long ldx, int C, long N, const float *b, const 
                        cudaStream_t st);
 void launch_zero_rows(float *x, long ldx, const int32_t *rows, int nrows, long N,
                       cudaStream_t st);
+/* have_ds: ds holds the block's td x fd downsample already (here and in the two filters below) */
 void launch_kadane(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
-                   long wnlimit, float *ds, int32_t *ranges, cudaStream_t st);
+                   long wnlimit, float *ds, int32_t *ranges, bool have_ds, cudaStream_t st);
 /* kadaneT: maximum-sum band along frequency per downsampled sample; ranges [Nds][4]
  * (channel start,end of the positive and negative band, -1 if not zapped). */
 void launch_kadaneT(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
-                    long bwlimit, float *ds, int32_t *ranges, cudaStream_t st);
+                    long bwlimit, float *ds, int32_t *ranges, bool have_ds, cudaStream_t st);
 /* mask: pixels of the td x fd downsampled block outside [Q1 - t*R, Q3 + t*R] are zapped;
  * sel: device scratch of MASK_SEL_WORDS words (selection state, then Q1, Q3 and the two
  * limits as float bits); nzap: device int receiving the number of zapped pixels. */
 constexpr int MASK_SEL_WORDS = 2 * 256 + 8;
 void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr, float *ds,
-                 uint32_t *sel, int32_t *nzap, cudaStream_t st);
+                 uint32_t *sel, int32_t *nzap, bool have_ds, cudaStream_t st);
 /* zp: C (mean, 1/sd) pairs of scratch */
 void launch_zdot(float *x, long ldx, int C, long N, float *s, double *sstats, float2 *zp,
                  cudaStream_t st);

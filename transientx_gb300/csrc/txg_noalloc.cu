@@ -66,7 +66,7 @@ extern "C" int txg_kadaneF_noalloc(float *x, int64_t ldx, int32_t nchans, int64_
         scratch = g_scratch[dev];
     }
     txg::launch_kadane(x, (long)ldx, nchans, (long)nsamples, td, fd, thr2, (long)wnlimit, scratch,
-                       ranges, (cudaStream_t)stream);
+                       ranges, false, (cudaStream_t)stream);
     TXG_CUDA_TRY(cudaGetLastError());
     return TXG_OK;
 }

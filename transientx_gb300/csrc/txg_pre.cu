@@ -38,140 +38,159 @@ __device__ __forceinline__ long long warp_sum_ll(long long v)
     return v;
 }
 
-/* r[i] = f(r[i], i) over a row by one warp, 16-byte accesses when the row is aligned, four
- * of them in flight per lane (each element is independent, so the access width does not
- * change any result). */
-template <typename F>
-__device__ __forceinline__ void row_map(float *__restrict__ r, long n, int lane, F f)
-{
-    long i0 = 0;
-    if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-        const long n4 = n / 4;
-        float4 *r4 = reinterpret_cast<float4 *>(r);
-        long q = lane;
-        for (; q + 3 * 32 < n4; q += 4 * 32) {
-            float4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = r4[q + 32 * u];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const long b = 4 * (q + 32 * u);
-                v[u].x = f(v[u].x, b);
-                v[u].y = f(v[u].y, b + 1);
-                v[u].z = f(v[u].z, b + 2);
-                v[u].w = f(v[u].w, b + 3);
-                r4[q + 32 * u] = v[u];
-            }
-        }
-        for (; q < n4; q += 32) {
-            float4 v = r4[q];
-            v.x = f(v.x, 4 * q);
-            v.y = f(v.y, 4 * q + 1);
-            v.z = f(v.z, 4 * q + 2);
-            v.w = f(v.w, 4 * q + 3);
-            r4[q] = v;
-        }
-        i0 = 4 * n4;
-    }
-    for (long i = i0 + lane; i < n; i += 32) r[i] = f(r[i], i);
-}
-
-struct Ident {
-    __device__ __forceinline__ float operator()(float v) const { return v; }
-};
-
 /* v -> (v - m) * inv, the per-channel standardisation of equalize and zdot */
 struct Standardise {
     float m, inv;
     __device__ __forceinline__ float operator()(float v) const { return __fmul_rn(__fsub_rn(v, m), inv); }
 };
 
-/* Two fixed-pattern reductions of one row by one warp: lane l takes i = l, l+32, l+64, ... in
- * runs of RED_RUN summed in FP32, adds each run total to its FP64 accumulator, and the lanes
- * combine by an xor butterfly.  MODE 1 -> (sum x, sum x*x), MODE 2 -> (sum x, sum x*y),
- * x = f(stored value).  Long runs keep the FP64 work (a small share of this part's arithmetic
- * rate) to two additions per 32 elements of a lane. */
+/* Two fixed-pattern reductions of one row: lane l of 32 takes i = l, l+32, l+64, ... in runs of
+ * RED_RUN summed in FP32, adds each run total to its FP64 accumulator, and the lanes combine by
+ * an xor butterfly.  MODE 1 -> (sum x, sum x*x), MODE 2 -> (sum x, sum x*y).  Long runs keep the
+ * FP64 work (a small share of this part's arithmetic rate) to two additions per 32 elements of a
+ * lane. */
 constexpr int RED_RUN = 32;
 
-template <int MODE, typename F = Ident>
-__device__ __forceinline__ void red32x2(const float *__restrict__ x, const float *__restrict__ y,
-                                        long n, int lane, double &o1, double &o2, F f = F())
+/* They are computed by a CTA of RB_THREADS: the warps take the runs in turn and leave each lane's
+ * FP32 totals in shared memory, then the first two warps add them in FP64, a sum each, in run
+ * order, and combine the lanes.  A row per warp left short blocks with few warps (47 us for the fit of 256 channels) and
+ * long ones with so many rows in flight that their second pass came from DRAM again.  get(i): the
+ * row's i-th value; the two sums come back in every thread.  cv: the values, stored on the
+ * way when not null (shared memory). */
+constexpr int RB_THREADS = 256;
+constexpr int RB_RUNS = 64; /* run totals per sum staged at a time: rows of 65536 samples in one go */
+
+struct RedRow {
+    float run[2][RB_RUNS][32];
+    double sum[2];
+};
+
+template <int MODE, typename G>
+__device__ __forceinline__ void red_row(G get, const float *__restrict__ y, long n, float *cv, RedRow &sh,
+                                              double &o1, double &o2)
 {
-    double a1 = 0., a2 = 0.;
-    long i = lane;
-    for (; i + (RED_RUN - 1) * 32 < n; i += RED_RUN * 32) { /* full runs, eight loads at a time */
-        float r1 = 0.f, r2 = 0.f;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long nruns = (n + 32 * RED_RUN - 1) / (32 * RED_RUN);
+    double a = 0.;
+    for (long base = 0; base < nruns; base += RB_RUNS) {
+        const int nr = (int)min((long)RB_RUNS, nruns - base);
+        for (int q = w; q < nr; q += RB_THREADS / 32) {
+            const long i0 = (base + q) * 32 * RED_RUN + lane;
+            float r1 = 0.f, r2 = 0.f;
+            auto add = [&](float v, long i) {
+                if (cv) cv[i] = v;
+                r1 = __fadd_rn(r1, v);
+                r2 = __fadd_rn(r2, __fmul_rn(v, MODE == 1 ? v : y[i]));
+            };
+            if (i0 - lane + 32 * RED_RUN <= n) { /* a full run, sixteen loads at a time */
 #pragma unroll
-        for (int h = 0; h < RED_RUN / 8; h++) {
-            float v[8], q[8];
+                for (int h = 0; h < RED_RUN / 16; h++) {
+                    float v[16];
 #pragma unroll
-            for (int r = 0; r < 8; r++) {
-                v[r] = f(x[i + 32 * (8 * h + r)]);
-                q[r] = MODE == 1 ? v[r] : y[i + 32 * (8 * h + r)];
+                    for (int r = 0; r < 16; r++) v[r] = get(i0 + 32 * (16 * h + r));
+#pragma unroll
+                    for (int r = 0; r < 16; r++) add(v[r], i0 + 32 * (16 * h + r));
+                }
+            } else {
+                for (long i = i0; i < n; i += 32) add(get(i), i);
             }
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                r1 = __fadd_rn(r1, v[r]);
-                r2 = __fadd_rn(r2, __fmul_rn(v[r], q[r]));
-            }
+            sh.run[0][q][lane] = r1;
+            sh.run[1][q][lane] = r2;
         }
-        a1 = __dadd_rn(a1, (double)r1);
-        a2 = __dadd_rn(a2, (double)r2);
+        __syncthreads();
+        if (w < 2)
+            for (int q = 0; q < nr; q++) a = __dadd_rn(a, (double)sh.run[w][q][lane]); /* an empty run adds +0 */
+        __syncthreads();
     }
-    if (i < n) { /* the last, partial run */
-        float r1 = 0.f, r2 = 0.f;
-        for (; i < n; i += 32) {
-            const float v = f(x[i]);
-            r1 = __fadd_rn(r1, v);
-            r2 = __fadd_rn(r2, MODE == 1 ? __fmul_rn(v, v) : __fmul_rn(v, y[i]));
-        }
-        a1 = __dadd_rn(a1, (double)r1);
-        a2 = __dadd_rn(a2, (double)r2);
+    if (w < 2) {
+        a = warp_sum_d(a);
+        if (lane == 0) sh.sum[w] = a;
     }
-    o1 = warp_sum_d(a1);
-    o2 = warp_sum_d(a2);
+    __syncthreads();
+    o1 = sh.sum[0];
+    o2 = sh.sum[1];
 }
 
 /* ---- skewness/kurtosis channel zap ------------------------------------------------------ */
-/* Exact integer sums of (v-128)^p, p = 1..4, per raw channel: threads over channels (4 per
- * thread with 32-bit loads when aligned), time split over blockIdx.y; 64-bit integer atomics
- * make the totals independent of the order. */
-constexpr int SK_TCHUNK = 128;
+/* Exact integer sums of (v-128)^p, p = 1..4, per raw channel; 64-bit integer atomics make the
+ * totals independent of the order.  A thread takes four channels (one 32-bit load when aligned)
+ * of every eighth of SK_TCHUNK samples, in 32 bits: |sums| of the first three powers stay below
+ * 32 * 128^3 = 2^26, the fourth's below 2^28 a sample and are carried to 64 bits every eight.
+ * The eight time slices are added in shared memory, so a CTA adds to each total once.  (64-bit
+ * sums in every thread, 128 samples each: 33 us for 256 channels x 15625 samples, 506 us for
+ * 8192 x 62496; so 6 and 171.) */
+constexpr int SK_TCHUNK = 256;
+constexpr int SK_SLICES = 8;
 
-__global__ void __launch_bounds__(256) k_sk_sums(const uint8_t *__restrict__ raw, int C_raw, long n0,
-                                                int vec, unsigned long long *__restrict__ sums)
+__global__ void __launch_bounds__(32 * SK_SLICES) k_sk_sums(const uint8_t *__restrict__ raw, int C_raw, long n0,
+                                                            int vec, unsigned long long *__restrict__ sums)
 {
-    const int per = vec ? 4 : 1;
-    const long c0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) * per;
-    if (c0 >= C_raw) return;
-    const long t0 = (long)blockIdx.y * SK_TCHUNK, t1 = min(t0 + SK_TCHUNK, n0);
-    long long a[4][4] = {};
-#pragma unroll 8
-    for (long t = t0; t < t1; t++) {
-        int v[4];
+    __shared__ int part[SK_SLICES][3][32][4];
+    __shared__ unsigned long long part4[SK_SLICES][32][4];
+    const int lane = threadIdx.x, ty = threadIdx.y;
+    const long c0 = ((long)blockIdx.x * 32 + lane) * 4;
+    const long t0 = (long)blockIdx.y * SK_TCHUNK + ty, t1 = min((long)(blockIdx.y + 1) * SK_TCHUNK, n0);
+    const int nc = (int)max(0L, min(4L, C_raw - c0));
+    int a[3][4] = {};
+    unsigned long long a4[4] = {};
+    auto take = [&](int k, int v, unsigned &q) {
+        const int d = v - 128, d2 = d * d;
+        a[0][k] += d;
+        a[1][k] += d2;
+        a[2][k] += d2 * d;
+        q += (unsigned)d2 * (unsigned)d2;
+    };
+    for (long t = t0; t < t1 && nc > 0;) {
+        unsigned q[4] = {};
         if (vec) {
-            const uchar4 q = *reinterpret_cast<const uchar4 *>(raw + t * C_raw + c0);
-            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+            if (t + 7 * SK_SLICES < t1) {
+                uchar4 v[8];
+#pragma unroll
+                for (int r = 0; r < 8; r++)
+                    v[r] = *reinterpret_cast<const uchar4 *>(raw + (t + r * SK_SLICES) * C_raw + c0);
+#pragma unroll
+                for (int r = 0; r < 8; r++) {
+                    take(0, v[r].x, q[0]);
+                    take(1, v[r].y, q[1]);
+                    take(2, v[r].z, q[2]);
+                    take(3, v[r].w, q[3]);
+                }
+                t += 8 * SK_SLICES;
+            } else {
+                const uchar4 v = *reinterpret_cast<const uchar4 *>(raw + t * C_raw + c0);
+                take(0, v.x, q[0]);
+                take(1, v.y, q[1]);
+                take(2, v.z, q[2]);
+                take(3, v.w, q[3]);
+                t += SK_SLICES;
+            }
         } else {
-            v[0] = raw[t * C_raw + c0];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < nc) take(k, raw[t * C_raw + c0 + k], q[k]);
+            t += SK_SLICES;
         }
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (k < per) {
-                const long long d = v[k] - 128, d2 = d * d;
-                a[k][0] += d;
-                a[k][1] += d2;
-                a[k][2] += d2 * d;
-                a[k][3] += d2 * d2;
-            }
-        }
+        for (int k = 0; k < 4; k++) a4[k] += q[k];
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-        if (k < per)
+    for (int k = 0; k < 4; k++) {
 #pragma unroll
-            for (int p = 0; p < 4; p++)
-                atomicAdd(&sums[(size_t)p * C_raw + c0 + k], (unsigned long long)a[k][p]);
+        for (int p = 0; p < 3; p++) part[ty][p][lane][k] = a[p][k];
+        part4[ty][lane][k] = a4[k];
+    }
+    __syncthreads();
+    /* 32 x 4 channels of 4 powers over the CTA's threads */
+    for (int e = ty * 32 + lane; e < 4 * 128; e += 32 * SK_SLICES) {
+        const int p = e >> 7, l = e >> 2 & 31, k = e & 3;
+        const long c = ((long)blockIdx.x * 32 + l) * 4 + k;
+        if (c >= C_raw) continue;
+        unsigned long long tot = 0;
+#pragma unroll
+        for (int y = 0; y < SK_SLICES; y++)
+            tot += p < 3 ? (unsigned long long)(long long)part[y][p][l][k] : part4[y][l][k];
+        atomicAdd(&sums[(size_t)p * C_raw + c], tot);
+    }
 }
 
 /* Per channel: moments -> skewness and excess kurtosis (double, each operation rounded as
@@ -495,24 +514,24 @@ __global__ void __launch_bounds__(FT_J * 8) k_unpack_f32(const float *__restrict
     }
 }
 
-/* Equalize statistics of a float block (one warp per channel): the sums of the values and of
- * their squares in the fixed FP64 reduction pattern of red32x2, then the same mean, variance,
+/* Equalize statistics of a float block (one CTA per channel): the sums of the values and of
+ * their squares in the fixed FP64 reduction pattern of red_row, then the same mean, variance,
  * (mean, 1/sd) pair and live flag as the 8-bit path's exact integer sums give. */
-__global__ void __launch_bounds__(256) k_eq_params_f32(const float *__restrict__ x, long ldx, int C,
-                                                       long N, float2 *__restrict__ eqp,
-                                                       uint8_t *__restrict__ live)
+__global__ void __launch_bounds__(RB_THREADS) k_eq_params_f32(const float *__restrict__ x, long ldx, long N,
+                                                              float2 *__restrict__ eqp, uint8_t *__restrict__ live)
 {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= C) return;
+    __shared__ RedRow sh;
+    const int c = blockIdx.x;
+    const float *r = x + (long)c * ldx;
     double s1, s2;
-    red32x2<1>(x + (long)w * ldx, nullptr, N, lane, s1, s2);
-    if (lane == 0) {
+    red_row<1>([=](long i) { return r[i]; }, nullptr, N, nullptr, sh, s1, s2);
+    if (threadIdx.x == 0) {
         const double dn = (double)N;
         double mean = __ddiv_rn(s1, dn);
         double var = __dsub_rn(__ddiv_rn(s2, dn), __dmul_rn(mean, mean));
         double sd = var > 0. ? __dsqrt_rn(var) : 1.;
-        eqp[w] = make_float2(__double2float_rn(mean), __double2float_rn(__ddiv_rn(1., sd)));
-        if (live) live[w] = var > 0. ? 1 : 0;
+        eqp[c] = make_float2(__double2float_rn(mean), __double2float_rn(__ddiv_rn(1., sd)));
+        if (live) live[c] = var > 0. ? 1 : 0;
     }
 }
 
@@ -599,6 +618,61 @@ __global__ void k_eq_apply(float *__restrict__ x, long ldx, long N, const float2
     }
 }
 
+/* The td x fd downsample of kadaneF, kadaneT and mask (ds[i*Cds + j], the sum over k < fd, then
+ * t < TD, of x[j*fd+k][i*TD+t]) in 16-byte accesses, and with APPLY k_eq_apply's pass in the same
+ * go: the block is read once for both (8192 channels x 62496 samples: 1.1 ms of reads saved).  A
+ * CTA takes 32 x 32 sums and writes them along channels through shared memory. */
+template <int TD, bool APPLY>
+__global__ void __launch_bounds__(256) k_ds(float *__restrict__ x, long ldx, int C, long N, int fd, int Cds, long Nds,
+                                            const float2 *__restrict__ eqp, const float *__restrict__ b,
+                                            const uint8_t *__restrict__ live, float *__restrict__ ds)
+{
+    __shared__ float tile[32][33];
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const long i = (long)blockIdx.x * 32 + lane, i0 = i * TD;
+    const int j0 = blockIdx.y * 32;
+    const bool full = i0 + TD <= N;
+    float4 bv[TD / 4];
+#pragma unroll
+    for (int q = 0; q < TD / 4; q++)
+        bv[q] = APPLY && b && full ? reinterpret_cast<const float4 *>(b + i0)[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int jj = ty; jj < 32; jj += 8) {
+        float acc = 0.f;
+        const int r0 = (j0 + jj) * fd;
+#pragma unroll 4
+        for (int k = 0; k < fd; k++) {
+            if (r0 + k >= C) break;
+            float *r = x + (long)(r0 + k) * ldx + i0;
+            const float2 e = APPLY ? eqp[r0 + k] : make_float2(0.f, 1.f);
+            const Standardise f{e.x, e.y};
+            const bool sub = APPLY && b && live[r0 + k];
+            if (full) {
+#pragma unroll
+                for (int q = 0; q < TD / 4; q++) {
+                    float4 v = reinterpret_cast<const float4 *>(r)[q];
+                    if (APPLY) {
+                        v = make_float4(f(v.x), f(v.y), f(v.z), f(v.w));
+                        if (sub)
+                            v = make_float4(__fsub_rn(v.x, bv[q].x), __fsub_rn(v.y, bv[q].y), __fsub_rn(v.z, bv[q].z),
+                                            __fsub_rn(v.w, bv[q].w));
+                        reinterpret_cast<float4 *>(r)[q] = v;
+                    }
+                    acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+                }
+            } else if (APPLY) { /* the rest of the row is in no sum */
+                for (long t = 0; i0 + t < N; t++) r[t] = sub ? __fsub_rn(f(r[t]), b[i0 + t]) : f(r[t]);
+            }
+        }
+        tile[lane][jj] = acc;
+    }
+    __syncthreads();
+    for (int ii = ty; ii < 32; ii += 8) {
+        const long io = (long)blockIdx.x * 32 + ii;
+        if (io < Nds && j0 + lane < Cds) ds[io * Cds + j0 + lane] = tile[ii][lane];
+    }
+}
+
 /* ---- channel mean per sample (zero-DM series), sequential over channels ---------------- */
 /* Channel sum per sample, in a fixed order: the channels are cut into CSUM_BLK consecutive
  * blocks of ceil(C/CSUM_BLK); each block is summed sequentially from 0.0f (one warp per block,
@@ -660,16 +734,36 @@ __global__ void __launch_bounds__(32 * CSUM_BLK) k_colmean(const float *__restri
     }
 }
 
-__global__ void k_smooth(const float *__restrict__ z, long N, long nw, float *__restrict__ b)
+/* b[i] = mean of z over [i - nw/2, i + nw/2] within the block, each summed in order from its first
+ * sample.  The chain of additions is a thread's own; z goes through shared memory, so that it
+ * runs at the addition's latency (34 us for windows of 1563 samples straight from memory, 7 so). */
+constexpr int SM_T = 128, SM_CH = 4096;
+
+__global__ void __launch_bounds__(SM_T) k_smooth(const float *__restrict__ z, long N, long nw, float *__restrict__ b)
 {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    long h = nw / 2;
-    long lo = i - h < 0 ? 0 : i - h;
-    long hi = i + h > N - 1 ? N - 1 : i + h;
+    __shared__ float zs[SM_CH];
+    const long i0 = (long)blockIdx.x * SM_T, i = i0 + threadIdx.x;
+    const long h = nw / 2;
+    const long lo = max(0L, i - h), hi = min(N - 1, i + h);
+    const long c0 = max(0L, i0 - h), c1 = min(N, i0 + SM_T + h); /* what the CTA reads */
     float acc = 0.f;
-    for (long u = lo; u <= hi; u++) acc = __fadd_rn(acc, z[u]);
-    b[i] = __fdiv_rn(acc, (float)(hi - lo + 1));
+    for (long c = c0; c < c1; c += SM_CH) {
+        const int n = (int)min((long)SM_CH, c1 - c);
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += SM_T) zs[k] = z[c + k];
+        __syncthreads();
+        const int k0 = (int)max(0L, lo - c), k1 = (int)min((long)n, hi + 1 - c);
+        int k = k0;
+        for (; k + 16 <= k1; k += 16) {
+            float v[16];
+#pragma unroll
+            for (int r = 0; r < 16; r++) v[r] = zs[k + r];
+#pragma unroll
+            for (int r = 0; r < 16; r++) acc = __fadd_rn(acc, v[r]);
+        }
+        for (; k < k1; k++) acc = __fadd_rn(acc, zs[k]);
+    }
+    if (i < N) b[i] = __fdiv_rn(acc, (float)(hi - lo + 1));
 }
 
 /* x[j][i] -= b[i] on live channels, four samples per thread (16-byte accesses when the row
@@ -718,9 +812,13 @@ __global__ void k_kadane_ds(const float *__restrict__ x, long ldx, int Cds, long
     ds[i * Cds + j] = acc;
 }
 
-/* One thread per downsampled channel runs the maximum-sum scan over the positive and the
- * negated series in one pass (strictly larger sum replaces the best window; the running
- * sum restarts after it drops below zero), then applies the S/N test. */
+/* The maximum-sum scan of 32 downsampled channels by a CTA of two warps, one for the series and
+ * one for the negated series, a channel per lane (strictly larger sum replaces the best window;
+ * the running sum restarts after it drops below zero), then the S/N test.  A sample's chain is
+ * an addition and a maximum with zero (a NaN sum stays one, as a comparison with zero leaves
+ * it); the two warps share the staged tiles, so that the staging and the bookkeeping beside
+ * the chain are split over schedulers (both signs by one warp: 66 us for 64 channels x 1953
+ * samples, so 27). */
 constexpr int KS_T = 96; /* samples per staged tile in the kadaneF scan */
 constexpr int KS_NB = 4; /* tile buffers: three in flight while one is scanned */
 
@@ -733,78 +831,78 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;" ::: "memory"); }
 
-__global__ void __launch_bounds__(32) k_kadane_scan(const float *__restrict__ ds, int Cds, long Nds,
+__global__ void __launch_bounds__(64) k_kadane_scan(const float *__restrict__ ds, int Cds, int Nds,
                                                     int tdk, int fdk, float thr, long wnlimit,
                                                     int32_t *__restrict__ ranges)
 {
-    /* each lane copies (cp.async) and later reads only its own channel's column of the tiles,
-     * so no barrier is needed; a buffer is refilled only after the next tile's scan */
     __shared__ float tile[KS_NB][KS_T][32];
-    const int lane = threadIdx.x, j = blockIdx.x * 32 + lane;
-    float bestp = -INFINITY, bestn = -INFINITY, curp = 0.f, curn = 0.f;
-    long csp = 0, csn = 0, sp = 0, ep = -1, sn = 0, en = -1;
-    auto step = [&](long i, float v) {
-        curp = __fadd_rn(curp, v);
-        curn = __fadd_rn(curn, -v);
-        if (curp > bestp) { bestp = curp; sp = csp; ep = i; }
-        if (curn > bestn) { bestn = curn; sn = csn; en = i; }
-        if (curp < 0.f) { curp = 0.f; csp = i + 1; }
-        if (curn < 0.f) { curn = 0.f; csn = i + 1; }
+    const int lane = threadIdx.x & 31, neg = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
+    const unsigned flip = neg ? 0x80000000u : 0u;
+    float best = -INFINITY, cur = 0.f;
+    int cs = 0, sb = 0, eb = -1;
+    auto step = [&](int i, float v) {
+        cur = __fadd_rn(cur, __uint_as_float(__float_as_uint(v) ^ flip));
+        if (cur > best) {
+            best = cur;
+            sb = cs;
+            eb = i;
+        }
+        if (cur < 0.f) cs = i + 1;
+        asm("max.NaN.f32 %0, %0, 0f00000000;" : "+f"(cur));
     };
-    /* the warp's 32 channels are staged KS_T samples at a time (one coalesced 128-byte row per
-     * copy instruction), then each lane scans its channel sequentially */
-    const long ntl = (Nds + KS_T - 1) / KS_T;
-    auto stage = [&](long tl) {
+    /* the 32 channels are staged KS_T samples at a time (one coalesced 128-byte row per copy
+     * instruction), every other row by each warp */
+    const int ntl = (Nds + KS_T - 1) / KS_T;
+    auto stage = [&](int tl) {
         if (tl < ntl && j < Cds) {
-            const long t0 = tl * KS_T;
-            const int nt = (int)min((long)KS_T, Nds - t0);
-            float(*tb)[32] = tile[tl % KS_NB];
-            const float *src = ds + t0 * Cds + j;
-            for (int r = 0; r < nt; r++) cp_async4(&tb[r][lane], src + (long)r * Cds);
+            const int nt = min(KS_T, Nds - tl * KS_T);
+            const float *src = ds + (long)(tl * KS_T + neg) * Cds + j;
+            float *dst = &tile[tl % KS_NB][neg][lane];
+#pragma unroll 8
+            for (int r = neg; r < nt; r += 2, src += 2 * (long)Cds, dst += 64) cp_async4(dst, src);
         }
         cp_async_commit(); /* one group per tile, empty past the end */
     };
     stage(0);
     stage(1);
     stage(2);
-    for (long tl = 0; tl < ntl; tl++) {
-        cp_async_wait_2(); /* all but the two newest groups done: tile tl has landed */
-        if (j < Cds) {
-            const long t0 = tl * KS_T;
-            const int nt = (int)min((long)KS_T, Nds - t0);
-            const float(*tb)[32] = tile[tl % KS_NB];
+    for (int tl = 0; tl < ntl; tl++) {
+        cp_async_wait_2(); /* all but the two newest groups done */
+        __syncthreads();   /* tile tl has landed for both warps, tile tl-1 is read no more */
+        stage(tl + 3);     /* into the buffer of tile tl-1 */
+        const int t0 = tl * KS_T, nt = min(KS_T, Nds - t0);
+        const float(*tb)[32] = tile[tl % KS_NB];
+        if (nt == KS_T) {
+#pragma unroll 16
+            for (int r = 0; r < KS_T; r++) step(t0 + r, tb[r][lane]);
+        } else {
             for (int r = 0; r < nt; r++) step(t0 + r, tb[r][lane]);
         }
-        stage(tl + 3); /* into the buffer of tile tl-1 */
     }
     if (j >= Cds) return;
     const float var = (float)(tdk * fdk);
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-        float boxsum = p == 0 ? bestp : bestn;
-        long s = p == 0 ? sp : sn, e = p == 0 ? ep : en;
-        long wn = e - s + 1;
-        float snr2 = 0.f;
-        if (wn > wnlimit) snr2 = __fdiv_rn(__fmul_rn(boxsum, boxsum), __fmul_rn((float)wn, var));
-        bool zap = Nds > 0 && snr2 > thr;
-        ranges[4 * j + 2 * p] = zap ? (int32_t)(s * tdk) : -1;
-        ranges[4 * j + 2 * p + 1] = zap ? (int32_t)((e + 1) * tdk) : -1;
-    }
+    const long s = sb, e = eb, wn = e - s + 1;
+    float snr2 = 0.f;
+    if (wn > wnlimit) snr2 = __fdiv_rn(__fmul_rn(best, best), __fmul_rn((float)wn, var));
+    const bool zap = Nds > 0 && snr2 > thr;
+    ranges[4 * j + 2 * neg] = zap ? (int32_t)(s * tdk) : -1;
+    ranges[4 * j + 2 * neg + 1] = zap ? (int32_t)((e + 1) * tdk) : -1;
 }
 
-/* One CTA per channel row: zero its downsampled channel's zapped windows (only those
+/* One warp per channel row: zero its downsampled channel's zapped windows (only those
  * samples are touched). */
-__global__ void k_kadane_apply(float *__restrict__ x, long ldx, long N, int fdk,
-                               const int32_t *__restrict__ ranges)
+__global__ void __launch_bounds__(256) k_kadane_apply(float *__restrict__ x, long ldx, long N, int C, int fdk,
+                                                      const int32_t *__restrict__ ranges)
 {
-    const int jr = blockIdx.x;
+    const int jr = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (jr >= C) return;
     const int32_t *r = ranges + 4 * (jr / fdk);
     float *row = x + (long)jr * ldx;
 #pragma unroll
     for (int p = 0; p < 2; p++) {
         const long a = r[2 * p], b = min((long)r[2 * p + 1], N);
-        if (a < 0) continue;
-        for (long i = a + threadIdx.x; i < b; i += blockDim.x) row[i] = 0.f;
+        if (a >= 0)
+            for (long i = a + lane; i < b; i += 32) row[i] = 0.f;
     }
 }
 
@@ -945,27 +1043,26 @@ __global__ void k_mask_apply(float *__restrict__ x, long ldx, long N, int Cds, l
 }
 
 /* ---- zdot ------------------------------------------------------------------------------ */
-/* Per channel (one warp): mean and standard deviation of the row (fixed-pattern sums) ->
+/* Per channel (one CTA): mean and standard deviation of the row (fixed-pattern sums) ->
  * zp[j] = ((float)mean, (float)(1/sd)), sd = 1 when the variance is not positive.  The
  * standardised row is never stored: the channel mean and the fit recompute it. */
-__global__ void __launch_bounds__(256) k_zdot_norm(const float *__restrict__ x, long ldx, int C, long N,
-                                                   float2 *__restrict__ zp)
+__global__ void __launch_bounds__(RB_THREADS) k_zdot_norm(const float *__restrict__ x, long ldx, long N,
+                                                          float2 *__restrict__ zp)
 {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= C) return;
-    const float *r = x + (long)w * ldx;
+    __shared__ RedRow sh;
+    const float *r = x + (long)blockIdx.x * ldx;
     double s1, s2;
-    red32x2<1>(r, nullptr, N, lane, s1, s2);
-    if (lane == 0) {
+    red_row<1>([=](long i) { return r[i]; }, nullptr, N, nullptr, sh, s1, s2);
+    if (threadIdx.x == 0) {
         const double dn = (double)N;
         double mean = __ddiv_rn(s1, dn);
         double var = __dsub_rn(__ddiv_rn(s2, dn), __dmul_rn(mean, mean));
         double sd = var > 0. ? __dsqrt_rn(var) : 1.;
-        zp[w] = make_float2(__double2float_rn(mean), __double2float_rn(__ddiv_rn(1., sd)));
+        zp[blockIdx.x] = make_float2(__double2float_rn(mean), __double2float_rn(__ddiv_rn(1., sd)));
     }
 }
 
-/* se and ss of the zero-DM series in the fixed pattern of red32x2: lane l's runs of RED_RUN
+/* se and ss of the zero-DM series in the fixed pattern of red_row: lane l's runs of RED_RUN
  * elements (l + 32*(RED_RUN*rho + r)) are summed in FP32 by all threads at once, then each
  * lane adds its run totals in FP64 in run order and the lanes combine by the xor butterfly. */
 constexpr int SST_RUNS = 4096; /* run totals staged per lane set (2 floats each) */
@@ -1011,28 +1108,53 @@ __global__ void __launch_bounds__(1024) k_zdot_sstats(const float *__restrict__ 
     }
 }
 
-/* Per channel (one warp), on the standardised row n = (x - m)*inv: least-squares alpha, beta
- * of n on s, then x <- n - (alpha*s + beta). */
-__global__ void __launch_bounds__(256) k_zdot_fit(float *__restrict__ x, long ldx, int C, long N,
-                                                  const float2 *__restrict__ zp,
-                                                  const float *__restrict__ s,
-                                                  const double *__restrict__ sst)
+/* Per channel (one CTA), on the standardised row n = (x - m)*inv: least-squares alpha, beta of n
+ * on s, then x <- n - (alpha*s + beta).  CACHE: the standardised row stays in shared memory between
+ * the two (rows up to ZF_CACHE samples; a longer one's second read finds it in L2, the CTAs in
+ * flight holding a few dozen MB).  A warp per row took 47 us for 256 channels of 15625 samples and
+ * 3.7 ms for the five rows of 8192 channels; so 12 us and 2.8 ms. */
+constexpr long ZF_CACHE = 16384;
+
+template <bool CACHE>
+__global__ void __launch_bounds__(RB_THREADS) k_zdot_fit(float *__restrict__ x, long ldx, long N,
+                                                         const float2 *__restrict__ zp,
+                                                         const float *__restrict__ s,
+                                                         const double *__restrict__ sst)
 {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= C) return;
-    float *r = x + (long)w * ldx;
-    const Standardise nf{zp[w].x, zp[w].y};
+    extern __shared__ float row[];
+    __shared__ RedRow sh;
+    __shared__ float2 ab;
+    float *r = x + (long)blockIdx.x * ldx;
+    const float2 z = zp[blockIdx.x];
+    const Standardise nf{z.x, z.y};
     double xe, xs;
-    red32x2<2>(r, s, N, lane, xe, xs, nf);
-    const double se = sst[0], ss = sst[1], dn = (double)N;
-    double tmp = __dsub_rn(__dmul_rn(se, se), __dmul_rn(ss, dn));
-    double alpha = 0., beta = 0.;
-    if (tmp != 0.) {
-        alpha = __ddiv_rn(__dsub_rn(__dmul_rn(xe, se), __dmul_rn(xs, dn)), tmp);
-        beta = __ddiv_rn(__dsub_rn(__dmul_rn(xs, se), __dmul_rn(xe, ss)), tmp);
+    red_row<2>([=](long i) { return nf(r[i]); }, s, N, CACHE ? row : nullptr, sh, xe, xs);
+    if (threadIdx.x == 0) {
+        const double se = sst[0], ss = sst[1], dn = (double)N;
+        double tmp = __dsub_rn(__dmul_rn(se, se), __dmul_rn(ss, dn));
+        double alpha = 0., beta = 0.;
+        if (tmp != 0.) {
+            alpha = __ddiv_rn(__dsub_rn(__dmul_rn(xe, se), __dmul_rn(xs, dn)), tmp);
+            beta = __ddiv_rn(__dsub_rn(__dmul_rn(xs, se), __dmul_rn(xe, ss)), tmp);
+        }
+        ab = make_float2(__double2float_rn(alpha), __double2float_rn(beta));
     }
-    const float af = __double2float_rn(alpha), bf = __double2float_rn(beta);
-    row_map(r, N, lane, [=](float v, long i) { return __fsub_rn(nf(v), __fadd_rn(__fmul_rn(af, s[i]), bf)); });
+    __syncthreads();
+    const float af = ab.x, bf = ab.y;
+    auto out = [=](float n, float sv) { return __fsub_rn(n, __fadd_rn(__fmul_rn(af, sv), bf)); };
+    long i0 = 0;
+    if (((reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(s)) & 15) == 0) {
+        const long n4 = N / 4;
+#pragma unroll 4
+        for (long k = threadIdx.x; k < n4; k += RB_THREADS) {
+            float4 v = CACHE ? reinterpret_cast<const float4 *>(row)[k] : reinterpret_cast<const float4 *>(r)[k];
+            const float4 q = reinterpret_cast<const float4 *>(s)[k];
+            if (!CACHE) v = make_float4(nf(v.x), nf(v.y), nf(v.z), nf(v.w));
+            reinterpret_cast<float4 *>(r)[k] = make_float4(out(v.x, q.x), out(v.y, q.y), out(v.z, q.z), out(v.w, q.w));
+        }
+        i0 = 4 * n4;
+    }
+    for (long i = i0 + threadIdx.x; i < N; i += RB_THREADS) r[i] = out(CACHE ? row[i] : nf(r[i]), s[i]);
 }
 
 inline unsigned nblk(long n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -1046,9 +1168,8 @@ void launch_skzap(const uint8_t *raw, int C_raw, long n0, float thr, unsigned lo
 {
     cudaMemsetAsync(sums, 0, sizeof(unsigned long long) * 4 * (size_t)C_raw, st);
     const int vec = (C_raw % 4 == 0) && ((reinterpret_cast<uintptr_t>(raw) & 3) == 0);
-    const long per_thread = vec ? 4 : 1;
-    dim3 g1(nblk((C_raw + per_thread - 1) / per_thread, 256), nblk(n0, SK_TCHUNK));
-    k_sk_sums<<<g1, 256, 0, st>>>(raw, C_raw, n0, vec, sums);
+    dim3 g1(nblk(C_raw, 128), nblk(n0, SK_TCHUNK));
+    k_sk_sums<<<g1, dim3(32, SK_SLICES), 0, st>>>(raw, C_raw, n0, vec, sums);
     k_sk_stats<<<nblk(C_raw, 256), 256, 0, st>>>(sums, C_raw, n0, stats);
     k_sk_select<<<1, 1024, 0, st>>>(C_raw, thr, stats, mask);
 }
@@ -1104,7 +1225,45 @@ void launch_unpack_f32(const float *blk, int C_raw, long n0, int td, int fd, flo
 void launch_eq_params_f32(const float *x, long ldx, int C, long N, float2 *eqp, uint8_t *live,
                           cudaStream_t st)
 {
-    k_eq_params_f32<<<nblk((long)C * 32, 256), 256, 0, st>>>(x, ldx, C, N, eqp, live);
+    k_eq_params_f32<<<C, RB_THREADS, 0, st>>>(x, ldx, N, eqp, live);
+}
+
+/* k_ds where it applies (td 4, 8 or 16 and aligned rows): with eqp also the equalize apply. */
+static bool downsample(float *x, long ldx, int C, long N, int td, int fd, const float2 *eqp, const float *b,
+                       const uint8_t *live, float *ds, cudaStream_t st)
+{
+    if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(b)) & 15) != 0 || ldx % 4 != 0) return false;
+    const int Cds = C / fd;
+    const long Nds = N / td;
+    if (Cds < 1 || Nds < 1) return false;
+    /* with the apply, the samples and channels left over by td and fd are covered too */
+    const dim3 grid(nblk((N + td - 1) / td, 32), nblk((C + fd - 1) / fd, 32));
+    if (grid.y > 65535) return false;
+#define TXG_DS(TD)                                                                                     \
+    do {                                                                                               \
+        if (eqp)                                                                                       \
+            k_ds<TD, true><<<grid, 256, 0, st>>>(x, ldx, C, N, fd, Cds, Nds, eqp, b, live, ds);        \
+        else                                                                                           \
+            k_ds<TD, false><<<grid, 256, 0, st>>>(x, ldx, C, N, fd, Cds, Nds, nullptr, nullptr, nullptr, ds); \
+        return true;                                                                                   \
+    } while (0)
+    if (td == 4) TXG_DS(4);
+    if (td == 8) TXG_DS(8);
+    if (td == 16) TXG_DS(16);
+#undef TXG_DS
+    return false;
+}
+
+static void kadane_ds(float *x, long ldx, int Cds, long Nds, int C, long N, int td, int fd, float *ds, cudaStream_t st)
+{
+    if (!downsample(x, ldx, C, N, td, fd, nullptr, nullptr, nullptr, ds, st))
+        k_kadane_ds<<<dim3(nblk(Nds, 128), Cds), 128, 0, st>>>(x, ldx, Cds, Nds, td, fd, ds);
+}
+
+bool launch_eq_apply_ds(float *x, long ldx, int C, long N, const float2 *eqp, const float *b, const uint8_t *live,
+                        int td, int fd, float *ds, cudaStream_t st)
+{
+    return downsample(x, ldx, C, N, td, fd, eqp, b, live, ds, st);
 }
 
 void launch_eq_apply(float *x, long ldx, int C, long N, const float2 *eqp, const float *b,
@@ -1125,7 +1284,7 @@ void launch_colmean(const float *x, long ldx, int C, long N, const uint8_t *live
 
 void launch_smooth(const float *z, long N, long nw, float *b, cudaStream_t st)
 {
-    k_smooth<<<nblk(N, 128), 128, 0, st>>>(z, N, nw, b);
+    k_smooth<<<nblk(N, SM_T), SM_T, 0, st>>>(z, N, nw, b);
 }
 
 void launch_sub_series(float *x, long ldx, int C, long N, const float *b, const uint8_t *live,
@@ -1144,42 +1303,37 @@ void launch_zero_rows(float *x, long ldx, const int32_t *rows, int nrows, long N
 }
 
 void launch_kadane(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
-                   long wnlimit, float *ds, int32_t *ranges, cudaStream_t st)
+                   long wnlimit, float *ds, int32_t *ranges, bool have_ds, cudaStream_t st)
 {
     int Cds = C / fdk;
     long Nds = N / tdk;
     if (Cds <= 0) return;
-    if (Nds > 0) {
-        dim3 g1(nblk(Nds, 128), Cds);
-        k_kadane_ds<<<g1, 128, 0, st>>>(x, ldx, Cds, Nds, tdk, fdk, ds);
-    }
-    k_kadane_scan<<<nblk(Cds, 32), 32, 0, st>>>(ds, Cds, Nds, tdk, fdk, thr, wnlimit, ranges);
-    k_kadane_apply<<<Cds * fdk, 128, 0, st>>>(x, ldx, N, fdk, ranges);
+    if (Nds > 0 && !have_ds) kadane_ds(x, ldx, Cds, Nds, C, N, tdk, fdk, ds, st);
+    k_kadane_scan<<<nblk(Cds, 32), 64, 0, st>>>(ds, Cds, (int)Nds, tdk, fdk, thr, wnlimit, ranges);
+    k_kadane_apply<<<nblk(Cds * fdk, 8), 256, 0, st>>>(x, ldx, N, Cds * fdk, fdk, ranges);
 }
 
 void launch_kadaneT(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
-                    long bwlimit, float *ds, int32_t *ranges, cudaStream_t st)
+                    long bwlimit, float *ds, int32_t *ranges, bool have_ds, cudaStream_t st)
 {
     const int Cds = C / fdk;
     const long Nds = N / tdk;
     if (Cds <= 0 || Nds <= 0) return;
-    dim3 g1(nblk(Nds, 128), Cds);
-    k_kadane_ds<<<g1, 128, 0, st>>>(x, ldx, Cds, Nds, tdk, fdk, ds);
+    if (!have_ds) kadane_ds(x, ldx, Cds, Nds, C, N, tdk, fdk, ds, st);
     k_kadaneT_scan<<<nblk(Nds, 64), 64, 0, st>>>(ds, Cds, Nds, tdk, fdk, thr, bwlimit, ranges);
     dim3 g3(nblk(N, 256), Cds * fdk);
     k_kadaneT_apply<<<g3, 256, 0, st>>>(x, ldx, N, tdk, Nds, ranges);
 }
 
 void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr, float *ds,
-                 uint32_t *sel, int32_t *nzap, cudaStream_t st)
+                 uint32_t *sel, int32_t *nzap, bool have_ds, cudaStream_t st)
 {
     const int Cds = C / fdk;
     const long Nds = N / tdk;
     cudaMemsetAsync(nzap, 0, sizeof(int32_t), st);
     if (Cds <= 0 || Nds <= 0) return;
     const long n = (long)Cds * Nds;
-    dim3 g1(nblk(Nds, 128), Cds);
-    k_kadane_ds<<<g1, 128, 0, st>>>(x, ldx, Cds, Nds, tdk, fdk, ds);
+    if (!have_ds) kadane_ds(x, ldx, Cds, Nds, C, N, tdk, fdk, ds, st);
     cudaMemsetAsync(sel, 0, sizeof(uint32_t) * MASK_SEL_WORDS, st);
     /* ranks of the quartiles, as the channel zap takes them: sorted[n/4], sorted[n-1-n/4] */
     const uint32_t k0 = (uint32_t)(n / 4), k1 = (uint32_t)(n - 1 - n / 4);
@@ -1195,10 +1349,17 @@ void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
 void launch_zdot(float *x, long ldx, int C, long N, float *s, double *sstats, float2 *zp,
                  cudaStream_t st)
 {
-    k_zdot_norm<<<nblk((long)C * 32, 256), 256, 0, st>>>(x, ldx, C, N, zp);
+    k_zdot_norm<<<C, RB_THREADS, 0, st>>>(x, ldx, N, zp);
     k_colmean<true><<<nblk(N, 32), dim3(32, CSUM_BLK), 0, st>>>(x, ldx, C, N, nullptr, zp, s);
     k_zdot_sstats<<<1, 1024, 0, st>>>(s, N, sstats);
-    k_zdot_fit<<<nblk((long)C * 32, 256), 256, 0, st>>>(x, ldx, C, N, zp, s, sstats);
+    if (N <= ZF_CACHE) {
+        const size_t smem = (size_t)(N + 3) / 4 * 16;
+        /* per call: the attribute belongs to the current device */
+        cudaFuncSetAttribute(k_zdot_fit<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ZF_CACHE * sizeof(float)));
+        k_zdot_fit<true><<<C, RB_THREADS, smem, st>>>(x, ldx, N, zp, s, sstats);
+    } else {
+        k_zdot_fit<false><<<C, RB_THREADS, 0, st>>>(x, ldx, N, zp, s, sstats);
+    }
 }
 
 } // namespace txg
