@@ -48,7 +48,7 @@ def _run(cmd: list[str]) -> None:
 
 def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, "txg_internal.h"),
+    headers = [os.path.join(CSRC, "txg_internal.h"), os.path.join(CSRC, "txg_device.cuh"),
                os.path.join(os.path.dirname(PKG), "include", "transientx_gb300.h")]
     jobs, objs = [], []
     nv = nvcc()

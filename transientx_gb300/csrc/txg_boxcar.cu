@@ -19,6 +19,7 @@
 #include <climits>
 #include <cstdlib>
 
+#include "txg_device.cuh"
 #include "txg_internal.h"
 
 namespace txg {
@@ -33,15 +34,6 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr size_t BX_SMEM_MAX = 200 * 1024; /* longest row kept whole */
 constexpr size_t BX_SMEM_TOP = 216 * 1024; /* with its bounds; + ~10 KB static stays under 227 KB */
 constexpr int BX_RUN = 32; /* row statistics: FP32 runs per thread before each FP64 addition */
-
-/* The exact double of a float by integer operations: a conversion, like every FP64 instruction,
- * holds a scheduler's FP64 unit for about 60 cycles on this part. */
-__device__ __forceinline__ double f2d(float f)
-{
-    const unsigned u = __float_as_uint(f), mag = u & 0x7fffffffu;
-    if (mag - 0x00800000u >= 0x7f000000u && mag) return (double)f; /* subnormal, infinite, NaN */
-    return __hiloint2double((int)((u & 0x80000000u) | (mag ? (mag >> 3) + 0x38000000u : 0u)), (int)(u << 29));
-}
 
 /* Block sums of a and b in every thread: an xor butterfly in each warp, then over the warps.  The
  * lower half of a warp reduces a and the upper half b, so each level is one addition for both

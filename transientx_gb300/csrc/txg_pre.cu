@@ -16,6 +16,7 @@
 
 #include <algorithm>
 
+#include "txg_device.cuh"
 #include "txg_internal.h"
 
 namespace txg {
@@ -53,9 +54,9 @@ constexpr int RED_RUN = 32;
 
 /* They are computed by a CTA of RB_THREADS: the warps take the runs in turn and leave each lane's
  * FP32 totals in shared memory, then the first two warps add them in FP64, a sum each, in run
- * order, and combine the lanes.  A row per warp left short blocks with few warps (47 us for the fit of 256 channels) and
- * long ones with so many rows in flight that their second pass came from DRAM again.  get(i): the
- * row's i-th value; the two sums come back in every thread.  cv: the values, stored on the
+ * order, and combine the lanes.  A row per warp left short blocks with few warps (47 us for the
+ * fit of 256 channels) and long ones with so many rows in flight that their second pass came
+ * from DRAM again.  get(i): the row's i-th value; the two sums come back in every thread.  cv: the values, stored on the
  * way when not null (shared memory). */
 constexpr int RB_THREADS = 256;
 constexpr int RB_RUNS = 64; /* run totals per sum staged at a time: rows of 65536 samples in one go */
@@ -99,7 +100,7 @@ __device__ __forceinline__ void red_row(G get, const float *__restrict__ y, long
         }
         __syncthreads();
         if (w < 2)
-            for (int q = 0; q < nr; q++) a = __dadd_rn(a, (double)sh.run[w][q][lane]); /* an empty run adds +0 */
+            for (int q = 0; q < nr; q++) a = __dadd_rn(a, f2d(sh.run[w][q][lane])); /* an empty run adds +0 */
         __syncthreads();
     }
     if (w < 2) {

@@ -19,6 +19,7 @@
 #include <functional>
 #include <vector>
 
+#include "txg_device.cuh"
 #include "txg_internal.h"
 
 namespace txg {
@@ -46,16 +47,21 @@ inline unsigned nblk(long n, int b) { return (unsigned)((n + b - 1) / b); }
 /* ---- sequential per-row chains ----------------------------------------------------------- */
 /* The reference's statistics, running sums and kadane scans are chains: each sample's float or
  * double operation needs the previous one's result, so a row is one lane's work.  What need
- * not be serial is the memory side.  A warp takes 32 rows; RT-sample tiles of all 32 are
- * copied into shared memory by cp.async, one coalesced 128-byte row piece per instruction,
- * RNB - 1 tiles ahead of the scan, and each lane walks its own row of the tile (33-word pitch:
- * no bank conflicts).  The chain then runs at its arithmetic latency; a lane reading its row
- * straight from memory waited for an uncoalesced load at every sample (statistics of six
- * candidates of 1024 channels x 6640 samples: 3.8 ms a launch before, 0.71 ms so; boxcar
- * chains and search of 6 x 1024 rows of 1048 samples: 5.1 ms before, 0.61 + 0.23 ms). */
+ * not be serial is everything beside the chain.  A CTA of four warps takes 32 rows: warps 2 and 3
+ * copy RT-sample tiles of them into shared memory by cp.async, one coalesced 128-byte row piece
+ * per instruction, RNB - 1 tiles ahead, and prepare what the chains can be given ready (products,
+ * differences); warps 0 and 1 each run a chain, every lane along its own row of the tile
+ * (33-word pitch: no bank conflicts).  A chain then runs at its arithmetic's latency, about 5
+ * cycles a float and 60 a double operation (conversions included, hence f2d).  One thread per
+ * row straight from memory waited for an uncoalesced load at every sample; one warp per 32 rows
+ * doing all of it spent most of its issue slots on the staging.  Candidate of 256 channels x
+ * 2187 samples, us: zdot sums 1520 / 352 / 169, fit 1121 / 376 / 179, statistics (both) 1472 /
+ * 354 / 118, boxcar chains of 256 x 625 samples 3112 (with the search) / 364 / 221. */
 constexpr int RT = 32;
 constexpr int RNB = 4;
+constexpr int RP_THREADS = 128;
 typedef float RpTile[RT][RT + 1];
+typedef double RpTileD[RT][RT + 1];
 
 __device__ __forceinline__ void rp_cp4(float *dst, const float *src)
 {
@@ -66,83 +72,117 @@ __device__ __forceinline__ void rp_cp4(float *dst, const float *src)
 __device__ __forceinline__ void rp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void rp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(RNB - 2) : "memory"); }
 
-/* step(t, v) for t = 0 .. cnt-1 on every lane, v[k] = sample (start[k] + t) mod n of the lane's
- * row (start[k] + cnt <= 2n + 1); rows 0..nrow-1 at `rows` with `pitch`.  The lanes of a warp
- * call it together with the same cnt, n and nrow; lanes at or past nrow see undefined values.
- * tile: K * RNB tiles of the warp. */
-template <int K, typename Step>
-__device__ __forceinline__ void rp_scan(RpTile *tile, const float *rows, long pitch, int nrow, long n,
-                                        const long (&start)[K], long cnt, Step step)
+struct RpNone {
+    __device__ void operator()(int, int, int, float) const {}
+};
+struct RpNoTile {
+    __device__ void operator()(long, int) const {}
+};
+
+/* Walks samples t = 0 .. cnt-1 of 32 rows (nrow of them exist; the others' values are undefined):
+ * stream k's sample is (start + off[k] + t) mod n of the row, start = first[row] (shared memory,
+ * or 0 without), start + off[k] + cnt <= 3n.  prep(b, row, q, v) runs once for every sample of
+ * stream 0 on warps 2 and 3, before the chains come to it (b: tile parity, q: place in the
+ * tile); step(t, q, b, v) on both chain warps; after(tl, b) on warp 1 when warp 0 has finished
+ * tile tl.  tile: K * RNB tiles.  Starts and ends with a barrier. */
+template <int K, typename Prep, typename Step, typename After>
+__device__ __forceinline__ void rp_scan(RpTile *tile, const float *rows, long pitch, int nrow, long n, const int *first,
+                                        const long (&off)[K], long cnt, Prep prep, Step step, After after)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long ntl = (cnt + RT - 1) / RT;
     auto stage = [&](long tl) {
         if (tl < ntl) {
             const long t = tl * RT + lane;
+            const int b = (int)(tl % RNB);
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                RpTile &tb = tile[k * RNB + (int)(tl % RNB)];
+                if (first) {
 #pragma unroll 4
-                for (int r = 0; r < nrow; r++) {
-                    long i = __shfl_sync(0xffffffffu, start[k], r) + t;
+                    for (int r = (w - 2) * 16; r < min(nrow, (w - 1) * 16); r++) {
+                        long i = first[r] + off[k] + t;
+                        i = i >= n ? i - n : i;
+                        i = i >= n ? i - n : i;
+                        if (t < cnt) rp_cp4(&tile[k * RNB + b][r][lane], rows + r * pitch + i);
+                    }
+                } else {
+                    long i = off[k] + t;
                     i = i >= n ? i - n : i;
                     i = i >= n ? i - n : i;
-                    if (t < cnt) rp_cp4(&tb[r][lane], rows + r * pitch + i);
+                    const float *src = rows + (w - 2) * 16 * pitch + i;
+                    float *dst = &tile[k * RNB + b][(w - 2) * 16][lane];
+                    const int nr = min(nrow - (w - 2) * 16, 16);
+                    if (t < cnt)
+#pragma unroll 4
+                        for (int r = 0; r < nr; r++, src += pitch, dst += RT + 1) rp_cp4(dst, src);
                 }
             }
         }
         rp_commit(); /* one group per tile, empty past the end */
     };
-    __syncwarp(); /* the previous scan's tiles are read no more */
-#pragma unroll
-    for (int b = 0; b < RNB - 1; b++) stage(b);
+    __syncthreads(); /* the previous scan's tiles are read no more */
+    if (w >= 2)
+        for (int b = 0; b < RNB - 1; b++) stage(b);
     for (long tl = 0; tl < ntl; tl++) {
-        rp_wait();
-        __syncwarp(); /* every lane's copies of tile tl are there; tile tl-1 is read no more */
-        const long t0 = tl * RT;
-        const int b = (int)(tl % RNB);
-        float v[K];
-        if (t0 + RT <= cnt) {
-#pragma unroll 8
-            for (int q = 0; q < RT; q++) {
-#pragma unroll
-                for (int k = 0; k < K; k++) v[k] = tile[k * RNB + b][lane][q];
-                step(t0 + q, v);
-            }
+        const int b = (int)(tl % RNB), par = (int)(tl & 1);
+        if (w >= 2) {
+            rp_wait();
+            __syncwarp(); /* the warp's rows of tile tl are there */
+            for (int r = (w - 2) * 16; r < min(nrow, (w - 1) * 16); r++) prep(par, r, lane, tile[b][r][lane]);
+        }
+        __syncthreads(); /* tile tl is there for all; tile tl-1 is read no more */
+        if (w >= 2) {
+            stage(tl + RNB - 1);
         } else {
-            for (int q = 0; q < (int)(cnt - t0); q++) {
+            if (w == 1 && tl > 0) after(tl - 1, par ^ 1);
+            const long t0 = tl * RT;
+            const int nq = (int)min((long)RT, cnt - t0);
+            float v[K];
+            if (nq == RT) {
+#pragma unroll 8
+                for (int q = 0; q < RT; q++) {
 #pragma unroll
-                for (int k = 0; k < K; k++) v[k] = tile[k * RNB + b][lane][q];
-                step(t0 + q, v);
+                    for (int k = 0; k < K; k++) v[k] = tile[k * RNB + b][lane][q];
+                    step(t0 + q, q, par, v);
+                }
+            } else {
+                for (int q = 0; q < nq; q++) {
+#pragma unroll
+                    for (int k = 0; k < K; k++) v[k] = tile[k * RNB + b][lane][q];
+                    step(t0 + q, q, par, v);
+                }
             }
         }
-        stage(tl + RNB - 1);
     }
+    __syncthreads();
+    if (w == 1 && ntl > 0) after(ntl - 1, (int)((ntl - 1) & 1));
 }
 
-/* Candidate::zdot, first loop (candidate.cpp:837-859): per channel, double mean and (float
- * square) power; std 1 where it is 0. */
-__global__ void __launch_bounds__(32) k_rp_zdot_sums(const float *__restrict__ buf, const RpMeta *__restrict__ m,
-                                                     double *__restrict__ mean, double *__restrict__ std)
+/* Candidate::zdot, first loop (candidate.cpp:837-859): per channel, double mean (warp 0) and
+ * (float square) power (warp 1); std 1 where it is 0. */
+__global__ void __launch_bounds__(RP_THREADS) k_rp_zdot_sums(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                             double *__restrict__ mean, double *__restrict__ std)
 {
     __shared__ RpTile tile[RNB];
+    __shared__ double mean_sh[32];
     const RpMeta c = m[blockIdx.y];
-    const int j0 = blockIdx.x * 32, j = j0 + threadIdx.x;
+    const int j0 = blockIdx.x * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5, j = j0 + lane;
     if (j0 >= c.nchan) return;
-    double tmpmean = 0., tmpstd = 0.;
-    rp_scan<1>(tile, buf + c.off + (long)j0 * c.pitch, c.pitch, min(32, c.nchan - j0), c.nbin, {0}, c.nbin,
-               [&](long, const float(&v)[1]) {
-                   tmpmean += v[0];
-                   tmpstd += v[0] * v[0];
-               });
-    if (j >= c.nchan) return;
-    tmpmean /= c.nbin;
-    tmpstd /= c.nbin;
-    tmpstd -= tmpmean * tmpmean;
-    tmpstd = sqrt(tmpstd);
-    if (tmpstd == 0.) tmpstd = 1.;
-    mean[c.coff + j] = tmpmean;
-    std[c.coff + j] = tmpstd;
+    double acc = 0.;
+    rp_scan<1>(tile, buf + c.off + (long)j0 * c.pitch, c.pitch, min(32, c.nchan - j0), c.nbin, nullptr, {0}, c.nbin,
+               RpNone(), [&](long, int, int, const float(&v)[1]) { acc += f2d(w ? v[0] * v[0] : v[0]); }, RpNoTile());
+    acc /= c.nbin;
+    if (w == 0) mean_sh[lane] = acc;
+    __syncthreads();
+    if (j >= c.nchan || w > 1) return;
+    if (w == 0) {
+        mean[c.coff + j] = acc;
+    } else {
+        acc -= mean_sh[lane] * mean_sh[lane];
+        acc = sqrt(acc);
+        if (acc == 0.) acc = 1.;
+        std[c.coff + j] = acc;
+    }
 }
 
 /* its second half, one CTA per channel: x = (x - mean) / std in double, stored as float after
@@ -180,40 +220,47 @@ __global__ void k_rp_zdot_s(const float *__restrict__ buf, const RpMeta *__restr
     s[blockIdx.y * soff_stride + i] = acc;
 }
 
-/* zdot's least-squares fit (:866-885): the sums over each channel (xe, xs), and by the last CTA
- * of a candidate those of s (se, ss), which are the same for every channel */
-__global__ void __launch_bounds__(32) k_rp_zdot_fit(const float *__restrict__ buf, const RpMeta *__restrict__ m,
-                                                    const double *__restrict__ s_all, long soff_stride,
-                                                    double *__restrict__ xe_all, double *__restrict__ xs_all,
-                                                    double2 *__restrict__ ses)
+/* zdot's least-squares fit (:866-885): the sums over each channel, xe by warp 0 and xs by warp 1 from
+ * the products of warps 2 and 3; and by the last CTA of a candidate those of s, se and ss, which
+ * are the same for every channel (32 samples and squares read and formed at a time). */
+__global__ void __launch_bounds__(RP_THREADS) k_rp_zdot_fit(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                            const double *__restrict__ s_all, long soff_stride,
+                                                            double *__restrict__ xe_all, double *__restrict__ xs_all,
+                                                            double2 *__restrict__ ses)
 {
     __shared__ RpTile tile[RNB];
+    __shared__ RpTileD prod[2];
     const RpMeta c = m[blockIdx.y];
     const double *s = s_all + blockIdx.y * soff_stride;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (blockIdx.x == gridDim.x - 1) {
-        if (threadIdx.x == 0) {
-            double se = 0., ss = 0.;
-#pragma unroll 16
-            for (long i = 0; i < c.nbin; i++) {
-                const double v = s[i];
-                se += v;
-                ss += v * v;
-            }
-            ses[blockIdx.y] = make_double2(se, ss);
+        if (w > 1) return;
+        double acc = 0., v = lane < c.nbin ? s[lane] : 0.;
+        for (long i = 0; i < c.nbin; i += 32) {
+            const double p = w ? v * v : v;
+            v = i + 32 + lane < c.nbin ? s[i + 32 + lane] : 0.;
+            const int nq = (int)min(32L, c.nbin - i);
+            for (int q = 0; q < nq; q++) acc += __shfl_sync(0xffffffffu, p, q);
         }
+        if (lane == 0) (w ? ses[blockIdx.y].y : ses[blockIdx.y].x) = acc;
         return;
     }
-    const int j0 = blockIdx.x * 32, j = j0 + threadIdx.x;
+    const int j0 = blockIdx.x * 32, j = j0 + lane;
     if (j0 >= c.nchan) return;
-    double xe = 0., xs = 0.;
-    rp_scan<1>(tile, buf + c.off + (long)j0 * c.pitch, c.pitch, min(32, c.nchan - j0), c.nbin, {0}, c.nbin,
-               [&](long i, const float(&v)[1]) {
-                   xe += v[0];
-                   xs += v[0] * s[i];
-               });
+    double acc = 0., sv = 0.;
+    long tp = -1; /* the tile whose s the lane holds */
+    rp_scan<1>(tile, buf + c.off + (long)j0 * c.pitch, c.pitch, min(32, c.nchan - j0), c.nbin, nullptr, {0}, c.nbin,
+               [&](int par, int r, int q, float v) {
+                   if (r == (w - 2) * 16) { /* the warp's first row: the next tile */
+                       tp++;
+                       sv = tp * RT + q < c.nbin ? s[tp * RT + q] : 0.;
+                   }
+                   prod[par][r][q] = f2d(v) * sv;
+               },
+               [&](long, int q, int par, const float(&v)[1]) { acc += w ? prod[par][lane][q] : f2d(v[0]); }, RpNoTile());
     if (j >= c.nchan) return;
-    xe_all[c.coff + j] = xe;
-    xs_all[c.coff + j] = xs;
+    if (w == 0) xe_all[c.coff + j] = acc;
+    if (w == 1) xs_all[c.coff + j] = acc;
 }
 
 /* the fit's coefficients and its subtraction (:880-895), one CTA per channel */
@@ -242,75 +289,84 @@ __global__ void __launch_bounds__(256) k_rp_zdot_sub(float *__restrict__ buf, co
  * (circular), then over that window either skewness, kurtosis and lag-1 autocorrelation in
  * float (SHAPE, what azap reads) or mean and variance in double (what normalize reads). */
 template <bool SHAPE>
-__global__ void __launch_bounds__(32) k_rp_stats(const float *__restrict__ buf, const RpMeta *__restrict__ m,
-                                                 double *__restrict__ mean, double *__restrict__ var,
-                                                 float *__restrict__ skew, float *__restrict__ kurt,
-                                                 float *__restrict__ ac)
+__global__ void __launch_bounds__(RP_THREADS) k_rp_stats(const float *__restrict__ buf, const RpMeta *__restrict__ m,
+                                                         double *__restrict__ mean, double *__restrict__ var,
+                                                         float *__restrict__ skew, float *__restrict__ kurt,
+                                                         float *__restrict__ ac)
 {
     __shared__ RpTile tile[2 * RNB];
+    __shared__ int first[32];
+    __shared__ float shape[32];
+    __shared__ double mu_sh[32];
     const RpMeta c = m[blockIdx.y];
-    const int j0 = blockIdx.x * 32, j = j0 + threadIdx.x;
+    const int j0 = blockIdx.x * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5, j = j0 + lane;
     if (j0 >= c.nchan) return;
     const float *rows = buf + c.off + (long)j0 * c.pitch;
     const int nrow = min(32, c.nchan - j0);
     const long nbin = c.nbin, h = nbin / 2;
-    /* data_sumif starts at 0 and adds the data: 0.f + x */
+    /* data_sumif starts at 0 and adds the data: 0.f + x.  Both chain warps find the window. */
     float boxsum = 0.;
-    rp_scan<1>(tile, rows, c.pitch, nrow, nbin, {0}, h, [&](long, const float(&v)[1]) { boxsum += 0.f + v[0]; });
+    rp_scan<1>(tile, rows, c.pitch, nrow, nbin, nullptr, {0}, h, RpNone(),
+               [&](long, int, int, const float(&v)[1]) { boxsum += 0.f + v[0]; }, RpNoTile());
     float mn = boxsum;
     int istart = 0;
-    rp_scan<2>(tile, rows, c.pitch, nrow, nbin, {0, h}, nbin, [&](long i, const float(&v)[2]) {
-        boxsum -= 0.f + v[0];
-        boxsum += 0.f + v[1];
-        if (boxsum < mn) {
-            mn = boxsum;
-            istart = (int)i + 1;
-        }
-    });
+    rp_scan<2>(tile, rows, c.pitch, nrow, nbin, nullptr, {0, h}, nbin, RpNone(),
+               [&](long i, int, int, const float(&v)[2]) {
+                   boxsum -= 0.f + v[0];
+                   boxsum += 0.f + v[1];
+                   if (boxsum < mn) {
+                       mn = boxsum;
+                       istart = (int)i + 1;
+                   }
+               },
+               RpNoTile());
+    if (w == 0) first[lane] = istart;
     const long q = c.coff + j;
-    if (SHAPE) {
+    if (SHAPE) { /* warp 0: variance and skewness, warp 1: kurtosis and autocorrelation */
         const float tmp_mean = mn / h;
-        float tmp_var = 0., sk = 0., ku = 0., a1 = 0., last = 0;
-        rp_scan<1>(tile, rows, c.pitch, nrow, nbin, {(long)istart}, h, [&](long, const float(&v)[1]) {
-            const float t = (0.f + v[0]) - tmp_mean;
-            const float t2 = t * t, t3 = t2 * t, t4 = t3 * t;
-            tmp_var += t2;
-            sk += t3;
-            ku += t4;
-            a1 += t * last;
-            last = t;
-        });
-        tmp_var /= h;
+        float a = 0., b = 0., last = 0;
+        rp_scan<1>(tile, rows, c.pitch, nrow, nbin, first, {0}, h, RpNone(),
+                   [&](long, int, int, const float(&v)[1]) {
+                       const float t = (0.f + v[0]) - tmp_mean;
+                       const float t2 = t * t, t3 = t2 * t, t4 = t3 * t;
+                       a += w ? t4 : t2;
+                       b += w ? t * last : t3;
+                       last = t;
+                   },
+                   RpNoTile());
+        if (w == 0) shape[lane] = a / h; /* the variance */
+        __syncthreads();
+        if (w > 1 || j >= c.nchan) return;
+        const float tmp_var = shape[lane];
         if (tmp_var <= 0) {
-            sk = 0.;
-            ku = 0.;
-            a1 = 0.;
+            if (w) a = 0.;
+            b = 0.;
         }
-        sk /= h;
-        sk /= tmp_var * sqrtf(tmp_var);
-        ku /= h;
-        ku /= tmp_var * tmp_var;
-        ku -= 3.;
-        a1 /= h - 1;
-        a1 /= tmp_var;
-        if (j < c.nchan) {
+        if (w == 0) {
+            float sk = b;
+            sk /= h;
+            sk /= tmp_var * sqrtf(tmp_var);
             skew[q] = sk;
+        } else {
+            float ku = a, a1 = b;
+            ku /= h;
+            ku /= tmp_var * tmp_var;
+            ku -= 3.;
+            a1 /= h - 1;
+            a1 /= tmp_var;
             kurt[q] = ku;
             ac[q] = a1;
         }
-    } else {
-        double mu = 0., v2 = 0.;
-        rp_scan<1>(tile, rows, c.pitch, nrow, nbin, {(long)istart}, h, [&](long, const float(&v)[1]) {
-            mu += v[0];
-            v2 += v[0] * v[0];
-        });
-        mu /= h;
-        v2 /= h;
-        v2 -= mu * mu;
-        if (j < c.nchan) {
-            mean[q] = mu;
-            var[q] = v2;
-        }
+    } else { /* warp 0: mean, warp 1: mean square */
+        double acc = 0.;
+        rp_scan<1>(tile, rows, c.pitch, nrow, nbin, first, {0}, h, RpNone(),
+                   [&](long, int, int, const float(&v)[1]) { acc += f2d(w ? v[0] * v[0] : v[0]); }, RpNoTile());
+        acc /= h;
+        if (w == 0) mu_sh[lane] = acc;
+        __syncthreads();
+        if (w > 1 || j >= c.nchan) return;
+        if (w == 0) mean[q] = acc;
+        else var[q] = acc - mu_sh[lane] * mu_sh[lane];
     }
 }
 
@@ -389,24 +445,25 @@ __global__ void __launch_bounds__(128) k_rp_kadane_ds(const float *__restrict__ 
 
 /* kadane<float> of the XLibs helpers as the reference tree's callers use it (a new maximum
  * needs a strictly larger sum, the running sum restarts after it drops below zero), on the
- * positive (z = 0) or the negated (z = 1) sums, then the S/N test with no minimum window
- * (replot_fil passes nwidth 0): ranges[4*channel + 2*z] = first and last-plus-one sample, -1
- * where nothing is zapped */
-__global__ void __launch_bounds__(32) k_rp_kadane_scan(const float *__restrict__ ds, const RpMeta *__restrict__ m,
-                                                       int td, int fd, float threshold, long dstride,
-                                                       long *__restrict__ ranges)
+ * positive sums by warp 0 and the negated ones by warp 1, then the S/N test with no minimum
+ * window (replot_fil passes nwidth 0): ranges[4*channel + 2*sign] = first and last-plus-one
+ * sample, -1 where nothing is zapped */
+__global__ void __launch_bounds__(RP_THREADS) k_rp_kadane_scan(const float *__restrict__ ds,
+                                                               const RpMeta *__restrict__ m, int td, int fd,
+                                                               float threshold, long dstride, long *__restrict__ ranges)
 {
     __shared__ RpTile tile[RNB];
     const RpMeta c = m[blockIdx.y];
     const long nsds = c.nbin / td, ncds = c.nchan / fd;
-    const long j0 = (long)blockIdx.x * 32, j = j0 + threadIdx.x;
+    const int w = threadIdx.x >> 5;
+    const long j0 = (long)blockIdx.x * 32, j = j0 + (threadIdx.x & 31);
     if (j0 >= ncds) return;
-    const bool neg = blockIdx.z;
     float best = -INFINITY, cur = 0;
     int cs = 0, start = 0, end = -1;
-    rp_scan<1>(tile, ds + (c.coff + j0) * dstride, dstride, (int)min(32L, ncds - j0), max(nsds, 1L), {0}, nsds,
-               [&](long i, const float(&v)[1]) {
-                   cur = cur + (neg ? -v[0] : v[0]);
+    rp_scan<1>(tile, ds + (c.coff + j0) * dstride, dstride, (int)min(32L, ncds - j0), max(nsds, 1L), nullptr, {0}, nsds,
+               RpNone(),
+               [&](long i, int, int, const float(&v)[1]) {
+                   cur = cur + (w ? -v[0] : v[0]);
                    if (cur > best) {
                        best = cur;
                        start = cs;
@@ -416,14 +473,15 @@ __global__ void __launch_bounds__(32) k_rp_kadane_scan(const float *__restrict__
                        cur = 0;
                        cs = (int)i + 1;
                    }
-               });
-    if (j >= ncds) return;
+               },
+               RpNoTile());
+    if (j >= ncds || w > 1) return;
     const float var = (float)(td * fd);
     const long wn = (long)end - start + 1;
     float snr2 = 0.;
     if (wn > 0) snr2 = best * best / (wn * var);
     const bool zap = snr2 > threshold * threshold;
-    long *o = ranges + 4 * (c.coff + j) + 2 * blockIdx.z;
+    long *o = ranges + 4 * (c.coff + j) + 2 * w;
     o[0] = zap ? (long)start * td : -1;
     o[1] = zap ? (long)(end + 1) * td : -1;
 }
@@ -518,43 +576,51 @@ __global__ void k_rp_profile(const float *__restrict__ buf, float *__restrict__ 
 }
 
 /* The chains of matched_filter / peak_search (:1000-1030, :1131-1150): per row the double mean
- * and variance (get_mean_var), then twice round the row the float running sum of (x - mean),
- * each addition in double.  csum: 2*nbin floats per row, written through a shared-memory tile. */
-__global__ void __launch_bounds__(32) k_rp_csum(const float *__restrict__ h, const RpMeta *__restrict__ m,
-                                                const int *__restrict__ rows, double *__restrict__ var_all,
-                                                float *__restrict__ csump)
+ * (warp 0) and mean square (warp 1; a float's square is exact in a double, so the fused multiply-add
+ * rounds like the separate ones), then twice round the row the float running sum of (x - mean),
+ * each addition in double: warps 2 and 3 form the differences, warp 0 adds, warp 1 writes the
+ * finished tile.  csum: 2*nbin floats per row. */
+__global__ void __launch_bounds__(RP_THREADS) k_rp_csum(const float *__restrict__ h, const RpMeta *__restrict__ m,
+                                                        const int *__restrict__ rows, double *__restrict__ var_all,
+                                                        float *__restrict__ csump)
 {
     __shared__ RpTile tile[RNB];
-    __shared__ RpTile outt;
+    __shared__ RpTileD diff[2];
+    __shared__ RpTile outt[2];
+    __shared__ double mean_sh[32];
     const RpMeta c = m[blockIdx.y];
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long j0 = (long)blockIdx.x * 32, j = j0 + lane;
     if (j0 >= rows[blockIdx.y]) return;
     const long nbin = c.nbin;
     const int nrow = (int)min(32L, rows[blockIdx.y] - j0);
     const float *tim = h + c.hoff + j0 * nbin;
     float *cs = csump + (c.hoff + j0 * nbin) * 2;
-    double s1 = 0., s2 = 0.;
-    rp_scan<1>(tile, tim, nbin, nrow, nbin, {0}, nbin, [&](long, const float(&x)[1]) {
-        const double v = x[0];
-        s1 += v;
-        s2 += v * v;
-    });
-    const double mean = s1 / nbin, var = s2 / nbin - mean * mean;
-    if (lane < nrow) var_all[c.rowoff + j] = var;
+    double acc = 0.;
+    rp_scan<1>(tile, tim, nbin, nrow, nbin, nullptr, {0}, nbin, RpNone(),
+               [&](long, int, int, const float(&x)[1]) {
+                   const double v = f2d(x[0]);
+                   acc = w ? __fma_rn(v, v, acc) : acc + v;
+               },
+               RpNoTile());
+    acc /= nbin;
+    if (w == 0) mean_sh[lane] = acc;
+    __syncthreads();
+    if (w == 1 && lane < nrow) var_all[c.rowoff + j] = acc - mean_sh[lane] * mean_sh[lane];
     float csum = 0.;
-    rp_scan<1>(tile, tim, nbin, nrow, nbin, {0}, 2 * nbin, [&](long i, const float(&x)[1]) {
-        csum += x[0] - mean;
-        const int q = (int)(i % RT);
-        outt[lane][q] = csum;
-        if (q == RT - 1 || i == 2 * nbin - 1) {
-            __syncwarp();
-            if (lane <= q)
+    rp_scan<1>(tile, tim, nbin, nrow, nbin, nullptr, {0}, 2 * nbin,
+               [&](int par, int r, int q, float v) { diff[par][r][q] = f2d(v) - mean_sh[r]; },
+               [&](long, int q, int par, const float(&)[1]) {
+                   if (w) return;
+                   csum = (float)(f2d(csum) + diff[par][lane][q]);
+                   outt[par][lane][q] = csum;
+               },
+               [&](long tl, int par) {
+                   const long t = tl * RT + lane;
+                   if (t < 2 * nbin)
 #pragma unroll 4
-                for (int r = 0; r < nrow; r++) cs[r * 2 * nbin + i - q + lane] = outt[r][lane];
-            __syncwarp();
-        }
-    });
+                       for (int r = 0; r < nrow; r++) cs[r * 2 * nbin + t] = outt[par][r][lane];
+               });
 }
 
 /* best of a row or candidate: the first largest S in row-major order (the scan of :1065-1078) */
@@ -830,7 +896,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         for (auto &h : H) mc = std::max(mc, h.nchan);
         return mc;
     };
-    auto per32 = [&](int rows) { return nblk(rows, 32); }; /* warps of the row scans */
+    auto per32 = [&](int rows) { return nblk(rows, 32); }; /* CTAs of the row scans */
     auto maxelem = [&]() {
         long me = 0;
         for (auto &h : H) me = std::max(me, (long)h.nchan * h.nbin);
@@ -848,17 +914,17 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(mem.alloc(&xe, tchan));
         RP_TRY(mem.alloc(&xs, tchan));
         RP_TRY(mem.alloc(&ses, n));
-        k_rp_zdot_sums<<<dim3(per32(maxchan()), NB), 32, 0, st>>>(buf[cur], dmeta, mean, var);
+        k_rp_zdot_sums<<<dim3(per32(maxchan()), NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, mean, var);
         k_rp_zdot_norm<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
         k_rp_zdot_s<<<dim3(nblk(maxnbin, 64), NB), 64, 0, st>>>(buf[cur], dmeta, zs, maxnbin);
-        k_rp_zdot_fit<<<dim3(per32(maxchan()) + 1, NB), 32, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
+        k_rp_zdot_fit<<<dim3(per32(maxchan()) + 1, NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
         k_rp_zdot_sub<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
         RP_TRY(cudaGetLastError());
     }
     /* 2: get_stats (their skewness, kurtosis, autocorrelation drive azap) */
     std::vector<float> sk_h(tchan), ku_h(tchan), ac_h(tchan);
     if (upto >= 2) {
-        k_rp_stats<true><<<dim3(per32(maxchan()), NB), 32, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
+        k_rp_stats<true><<<dim3(per32(maxchan()), NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
         RP_TRY(cudaGetLastError());
         RP_TRY(cudaMemcpyAsync(sk_h.data(), skew, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
         RP_TRY(cudaMemcpyAsync(ku_h.data(), kurt, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
@@ -942,7 +1008,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
     }
     /* 7, 8: get_stats, normalize */
     if (upto >= 7)
-        k_rp_stats<false><<<dim3(per32(maxchan()), NB), 32, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
+        k_rp_stats<false><<<dim3(per32(maxchan()), NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
     if (upto >= 8)
         k_rp_normalize<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
     RP_TRY(cudaGetLastError());
@@ -967,8 +1033,8 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             RP_TRY(mem.alloc(&ds, (size_t)tchan * dstride));
             RP_TRY(mem.alloc(&rng, (size_t)tchan * 4));
             k_rp_kadane_ds<<<dim3(ncmax, NB), 128, 0, st>>>(buf[cur], dmeta, td, fd, ds, dstride);
-            k_rp_kadane_scan<<<dim3(per32((int)ncmax), NB, 2), 32, 0, st>>>(ds, dmeta, td, fd, (float)o->kadane[2],
-                                                                          dstride, rng);
+            k_rp_kadane_scan<<<dim3(per32((int)ncmax), NB), RP_THREADS, 0, st>>>(ds, dmeta, td, fd,
+                                                                                 (float)o->kadane[2], dstride, rng);
             k_rp_kadane_apply<<<dim3(maxchan(), NB), 128, 0, st>>>(buf[cur], dmeta, fd, rng);
             RP_TRY(cudaGetLastError());
         }
@@ -1107,7 +1173,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(mem.alloc(&dvar, nrows));
         RP_TRY(mem.alloc(&drbest, nrows));
         RP_TRY(mem.alloc(&dbest, n));
-        k_rp_csum<<<dim3(per32(maxrows), NB), 32, 0, st>>>(hb[hc], dmeta, drows, dvar, csump);
+        k_rp_csum<<<dim3(per32(maxrows), NB), RP_THREADS, 0, st>>>(hb[hc], dmeta, drows, dvar, csump);
         k_rp_match<<<dim3(maxrows, NB), 256, 0, st>>>(dmeta, drows, dvwn, dnbox, wstride, dvar, csump, dsnr, dwidm,
                                                      drbest);
         k_rp_best<<<NB, 256, 0, st>>>(dmeta, drows, drbest, dbest);
