@@ -19,7 +19,7 @@ CU_SRC = ["txg_pre.cu", "txg_dedisp.cu", "txg_boxcar.cu", "txg_api.cu", "txg_noa
 # files whose device arithmetic follows the reference's mixed float/double expressions as
 # written: no multiply-add contraction anywhere in them
 NO_FMAD = {"txg_replot.cu"}
-CPP_SRC = ["txg_plan.cpp", "txg_cluster.cpp"]
+CPP_SRC = ["txg_plan.cpp", "txg_cluster.cpp", "txg_xfer.cpp"]
 
 
 def nvcc() -> str:

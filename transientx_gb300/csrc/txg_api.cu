@@ -322,7 +322,11 @@ template <typename T> int dalloc(txg_handle *h, T **p, size_t count)
     void *q = nullptr;
     size_t bytes = count * sizeof(T);
     if (bytes == 0) bytes = 16;
-    TXG_CUDA_TRY(cudaMalloc(&q, bytes));
+    if (cudaMalloc(&q, bytes) != cudaSuccess) { /* what the scratch pool keeps may be enough */
+        cudaGetLastError();
+        scratch_trim();
+        TXG_CUDA_TRY(cudaMalloc(&q, bytes));
+    }
     h->allocs.push_back(q);
     TXG_CUDA_TRY(cudaMemsetAsync(q, 0, bytes, h->st));
     *p = (T *)q;
@@ -1056,6 +1060,7 @@ void txg_destroy(txg_handle *h)
     if (!h) return;
     free_all(h);
     delete h;
+    scratch_trim();
 }
 
 int txg_push_block_device(txg_handle *h, int32_t beam, const uint8_t *dev, int64_t nsamp)
@@ -1083,7 +1088,7 @@ int txg_push_block(txg_handle *h, int32_t beam, const uint8_t *host, int64_t nsa
     if (!pinned) {
         /* the staging buffer's previous copy (two blocks ago) must be done */
         TXG_CUDA_TRY(cudaEventSynchronize(h->raw_loaded[i]));
-        memcpy(h->stage[i], host, bytes);
+        host_copy(h->stage[i], host, bytes);
         src = h->stage[i];
     }
     /* copy stream: wait until the kernels of two blocks ago are done with raw[i]; the kernel
@@ -1131,7 +1136,7 @@ int txg_push_block_f32(txg_handle *h, int32_t beam, const float *host, int64_t n
     const float *src = host;
     if (!pinned) {
         TXG_CUDA_TRY(cudaEventSynchronize(h->rawf_loaded[i]));
-        memcpy(h->stagef[i], host, count * sizeof(float));
+        host_copy(h->stagef[i], host, count * sizeof(float));
         src = h->stagef[i];
     }
     TXG_CUDA_TRY(cudaStreamWaitEvent(h->cst, h->rawf_free[i], 0));
@@ -1268,8 +1273,8 @@ int txg_get_dense(txg_handle *h, int32_t beam, int32_t row, float *mxS, int32_t 
     if (int jr = join_rows(h)) return jr; /* results of the row streams */
     TXG_CUDA_TRY(cudaStreamSynchronize(h->st));
     size_t cnt = (size_t)P.cfg.ndm * P.nout;
-    if (mxS) TXG_CUDA_TRY(cudaMemcpy(mxS, b.mxS, cnt * sizeof(float), cudaMemcpyDeviceToHost));
-    if (mxwn) TXG_CUDA_TRY(cudaMemcpy(mxwn, b.mxwn, cnt * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    if (mxS) TXG_CUDA_TRY(copy_out(mxS, b.mxS, cnt * sizeof(float)));
+    if (mxwn) TXG_CUDA_TRY(copy_out(mxwn, b.mxwn, cnt * sizeof(int32_t)));
     return TXG_OK;
 }
 
@@ -1282,8 +1287,7 @@ int txg_get_timdata(txg_handle *h, int32_t beam, int32_t row, int64_t idm0, int6
     if (!out || idm0 < 0 || count < 0 || idm0 + count > P.cfg.ndm) return fail(TXG_ERR_ARG, "DM range");
     if (int jr = join_rows(h)) return jr; /* results of the row streams */
     TXG_CUDA_TRY(cudaStreamSynchronize(h->st));
-    TXG_CUDA_TRY(cudaMemcpy(out, h->br[beam][row].tim + idm0 * P.nout, count * P.nout * sizeof(float),
-                            cudaMemcpyDeviceToHost));
+    TXG_CUDA_TRY(copy_out(out, h->br[beam][row].tim + idm0 * P.nout, count * P.nout * sizeof(float)));
     return TXG_OK;
 }
 
@@ -1589,8 +1593,7 @@ int txg_boxcar(const float *tim, int64_t ndm, int64_t nsamples, const int32_t *v
         return fail(TXG_ERR_UNSUPPORTED, "nsamples or the widest boxcar exceeds the boxcar kernels' limits");
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return fail(TXG_ERR_NODEVICE, "no CUDA device");
-    cudaStream_t st;
-    TXG_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    Scratch mem;
     float *dtim = nullptr, *dS = nullptr;
     int32_t *dwn = nullptr, *dvwn = nullptr;
     txg_cand *dc = nullptr;
@@ -1598,73 +1601,42 @@ int txg_boxcar(const float *tim, int64_t ndm, int64_t nsamples, const int32_t *v
     double *dscr = nullptr;
     const size_t cnt = (size_t)ndm * nsamples;
     const long ccap = cands ? (cap > 0 ? cap : 0) : 0;
-    int rc = TXG_OK;
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(st);
-        cudaFree(dtim);
-        cudaFree(dS);
-        cudaFree(dwn);
-        cudaFree(dvwn);
-        cudaFree(dc);
-        cudaFree(dcount);
-        cudaFree(dscr);
-        cudaStreamDestroy(st);
-    };
-    do {
-        cudaError_t e;
-        if ((e = cudaMalloc(&dtim, cnt * sizeof(float))) != cudaSuccess ||
-            (e = cudaMalloc(&dvwn, nw * sizeof(int32_t))) != cudaSuccess ||
-            (e = cudaMalloc(&dcount, 2 * sizeof(int))) != cudaSuccess ||
-            (e = cudaMalloc(&dscr, boxcar_scratch_doubles(ndm) * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&dc, (ccap > 0 ? ccap : 1) * sizeof(txg_cand))) != cudaSuccess ||
-            (mxS && (e = cudaMalloc(&dS, cnt * sizeof(float))) != cudaSuccess) ||
-            (mxS && (e = cudaMalloc(&dwn, cnt * sizeof(int32_t))) != cudaSuccess)) {
-            rc = set_cuda_error(e, "cudaMalloc", __FILE__, __LINE__);
-            break;
-        }
-        if ((e = cudaMemcpyAsync(dtim, tim, cnt * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(dvwn, vwn, nw * sizeof(int32_t), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-            (e = cudaMemsetAsync(dcount, 0, 2 * sizeof(int), st)) != cudaSuccess) {
-            rc = set_cuda_error(e, "copy-in", __FILE__, __LINE__);
-            break;
-        }
-        rc = launch_boxcar(dtim, nsamples, ndm, nsamples, dvwn, nw, maxwn, iqr,
+    TXG_CUDA_TRY(mem.open());
+    cudaStream_t st = mem.st;
+    TXG_CUDA_TRY(mem.alloc(&dtim, cnt));
+    TXG_CUDA_TRY(mem.alloc(&dvwn, (size_t)nw));
+    TXG_CUDA_TRY(mem.alloc(&dcount, (size_t)2));
+    TXG_CUDA_TRY(mem.alloc(&dscr, boxcar_scratch_doubles(ndm)));
+    TXG_CUDA_TRY(mem.alloc(&dc, (size_t)ccap));
+    if (mxS) {
+        TXG_CUDA_TRY(mem.alloc(&dS, cnt));
+        TXG_CUDA_TRY(mem.alloc(&dwn, cnt));
+    }
+    TXG_CUDA_TRY(cudaMemcpyAsync(dtim, tim, cnt * sizeof(float), cudaMemcpyHostToDevice, st));
+    TXG_CUDA_TRY(cudaMemcpyAsync(dvwn, vwn, nw * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    TXG_CUDA_TRY(cudaMemsetAsync(dcount, 0, 2 * sizeof(int), st));
+    int rc = launch_boxcar(dtim, nsamples, ndm, nsamples, dvwn, nw, maxwn, iqr,
                            (flags & TXG_FLAG_AVX2_TAIL) ? 1 : 0, thre, dc, dcount, ccap, dS, dwn,
                            dscr, dcount + 1, st);
-        if (rc) break;
-        if ((e = cudaGetLastError()) != cudaSuccess) {
-            rc = set_cuda_error(e, "boxcar launch", __FILE__, __LINE__);
-            break;
-        }
-        int hc[2] = {0, 0};
-        if ((e = cudaMemcpyAsync(hc, dcount, 2 * sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(st)) != cudaSuccess) {
-            rc = set_cuda_error(e, "boxcar", __FILE__, __LINE__);
-            break;
-        }
-        if (mxS) {
-            if ((e = cudaMemcpy(mxS, dS, cnt * sizeof(float), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-                (mxwn && (e = cudaMemcpy(mxwn, dwn, cnt * sizeof(int32_t), cudaMemcpyDeviceToHost)) != cudaSuccess)) {
-                rc = set_cuda_error(e, "copy-out", __FILE__, __LINE__);
-                break;
-            }
-        }
-        if (ncand) *ncand = hc[0];
-        if (cands && ccap > 0) {
-            long keep = std::min<long>(hc[0], ccap);
-            if (keep > 0 &&
-                (e = cudaMemcpy(cands, dc, keep * sizeof(txg_cand), cudaMemcpyDeviceToHost)) != cudaSuccess) {
-                rc = set_cuda_error(e, "copy-out", __FILE__, __LINE__);
-                break;
-            }
-            std::sort(cands, cands + keep, [](const txg_cand &x, const txg_cand &y) {
-                return x.idm != y.idm ? x.idm < y.idm : x.isamp < y.isamp;
-            });
-            if (hc[0] > ccap) rc = fail(TXG_ERR_OVERFLOW, "candidate buffer overflow");
-        }
-    } while (0);
-    cleanup();
-    return rc;
+    if (rc) return rc;
+    TXG_CUDA_TRY(cudaGetLastError());
+    int hc[2] = {0, 0};
+    TXG_CUDA_TRY(cudaMemcpyAsync(hc, dcount, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    TXG_CUDA_TRY(cudaStreamSynchronize(st));
+    if (mxS) {
+        TXG_CUDA_TRY(copy_out(mxS, dS, cnt * sizeof(float)));
+        if (mxwn) TXG_CUDA_TRY(copy_out(mxwn, dwn, cnt * sizeof(int32_t)));
+    }
+    if (ncand) *ncand = hc[0];
+    if (cands && ccap > 0) {
+        const long keep = std::min<long>(hc[0], ccap);
+        if (keep > 0) TXG_CUDA_TRY(copy_out(cands, dc, keep * sizeof(txg_cand)));
+        std::sort(cands, cands + keep, [](const txg_cand &x, const txg_cand &y) {
+            return x.idm != y.idm ? x.idm < y.idm : x.isamp < y.isamp;
+        });
+        if (hc[0] > ccap) return fail(TXG_ERR_OVERFLOW, "candidate buffer overflow");
+    }
+    return TXG_OK;
 }
 
 int txg_cluster(const txg_cand *cands, int64_t n, double dms, double ddm, double fmax, double fmin,

@@ -66,6 +66,28 @@ long cluster_run(const txg_cand *c, long n, double dms, double ddm, double fmax,
                  double tsamp, double radius, int maxncand, int minpts, int drop, int maxwn,
                  txg_cand *out, long cap);
 
+/* Copies and scratch memory (txg_xfer.cpp). */
+void host_copy(void *dst, const void *src, size_t n);
+cudaError_t copy_out(void *dst, const void *dev, size_t n); /* device to any host memory; waits */
+/* gives back what the current device's scratch pool keeps */
+void scratch_trim();
+/* A stream of its own and device memory for one call, on the current device; both end with it. */
+class Scratch {
+public:
+    Scratch() = default;
+    ~Scratch();
+    Scratch(const Scratch &) = delete;
+    Scratch &operator=(const Scratch &) = delete;
+    cudaError_t open();
+    template <typename T> cudaError_t alloc(T **p, size_t count) { return get((void **)p, count * sizeof(T)); }
+    cudaStream_t st = nullptr;
+
+private:
+    cudaError_t get(void **p, size_t bytes);
+    cudaMemPool_t pool_ = nullptr; /* null: from cudaMalloc */
+    std::vector<void *> ptr_;
+};
+
 /* ---- kernel launchers (txg_pre.cu, txg_dedisp.cu, txg_boxcar.cu) -------------------- */
 void launch_skzap(const uint8_t *raw, int C_raw, long n0, float thr, unsigned long long *sums,
                   double *stats, uint8_t *mask, cudaStream_t st);

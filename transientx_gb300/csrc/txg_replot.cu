@@ -788,24 +788,6 @@ void rp_quartiles(const float *v, int n, float &q1, float &q3)
     q3 = s[s.size() / 4];
 }
 
-struct DevBuf {
-    std::vector<void *> p;
-    ~DevBuf()
-    {
-        for (void *q : p) cudaFree(q);
-    }
-    template <typename T> cudaError_t alloc(T **out, size_t count)
-    {
-        void *q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-        if (e == cudaSuccess) {
-            p.push_back(q);
-            *out = (T *)q;
-        }
-        return e;
-    }
-};
-
 } // namespace
 
 extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands, int64_t n,
@@ -841,22 +823,19 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return set_cuda_error(cudaErrorNoDevice, "txg_replot", __FILE__, __LINE__);
 
-    DevBuf mem;
+    Scratch mem;
     float *buf[2] = {nullptr, nullptr}, *skew, *kurt, *ac, *w;
     double *mean, *var;
     int *delay;
     RpMeta *dmeta;
-    cudaStream_t st = nullptr;
     cudaError_t e = cudaSuccess;
 #define RP_TRY(x)                                                                  \
     do {                                                                           \
         e = (x);                                                                   \
-        if (e != cudaSuccess) {                                                    \
-            if (st) cudaStreamDestroy(st);                                         \
-            return set_cuda_error(e, #x, __FILE__, __LINE__);                      \
-        }                                                                          \
+        if (e != cudaSuccess) return set_cuda_error(e, #x, __FILE__, __LINE__);    \
     } while (0)
-    RP_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    RP_TRY(mem.open());
+    const cudaStream_t st = mem.st;
     RP_TRY(mem.alloc(&buf[0], total));
     RP_TRY(mem.alloc(&buf[1], total));
     RP_TRY(mem.alloc(&mean, tchan));
@@ -943,8 +922,6 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         nbin_new = (long)(std::ceil(nbin_new / factor) * factor);
         if (nbin_new < h.nbin) cut[b] = nbin_new;
         if (cut[b] < 4) {
-            cudaStreamSynchronize(st);
-            cudaStreamDestroy(st);
             return set_arg_error("the chop to 2*nw*width leaves fewer than 4 samples");
         }
     }
@@ -1195,7 +1172,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             long pos = 0;
             for (long b = 0; b < n && pos < snrmap_cap; b++) {
                 const long cnt = std::min(H[b].rows * H[b].nbin, (long)snrmap_cap - pos);
-                RP_TRY(cudaMemcpy(snrmap + pos, dsnr + H[b].hoff, sizeof(float) * cnt, cudaMemcpyDeviceToHost));
+                RP_TRY(copy_out(snrmap + pos, dsnr + H[b].hoff, sizeof(float) * cnt));
                 pos += cnt;
             }
         }
@@ -1224,7 +1201,6 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         }
     }
     RP_TRY(cudaStreamSynchronize(st));
-    cudaStreamDestroy(st);
 #undef RP_TRY
     return TXG_OK;
 }
