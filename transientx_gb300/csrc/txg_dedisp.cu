@@ -649,7 +649,12 @@ __device__ __forceinline__ void addp(float &lo_acc, float &hi_acc, uint32_t v, _
 /* Odd-aligned pair copy of a 16-bit window: o[k] = (e[2k+1], e[2k+2]) as one word. */
 __device__ __forceinline__ void build_odd(const uint32_t *e, uint32_t *o, long nwords, int tid, int nth)
 {
-    for (long k = tid; k < nwords; k += nth) o[k] = __byte_perm(e[k], e[k + 1], 0x5432);
+    for (int k = tid; k < nwords / 4; k += nth) {
+        const uint4 v = reinterpret_cast<const uint4 *>(e)[k];
+        const uint32_t n = e[4 * k + 4];
+        reinterpret_cast<uint4 *>(o)[k] = make_uint4(__byte_perm(v.x, v.y, 0x5432), __byte_perm(v.y, v.z, 0x5432),
+                                                     __byte_perm(v.z, v.w, 0x5432), __byte_perm(v.w, n, 0x5432));
+    }
 }
 
 /* ---- stage 2 ---------------------------------------------------------------------------- */
@@ -794,7 +799,11 @@ k_stage2(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long nou
 
 /* Stage 2 on a 16-bit ring, two consecutive samples per 32-bit shared-memory load: the
  * subband windows are held as even-aligned pairs (bulk copies) and odd-aligned pairs (built
- * in shared memory).  Same order of additions as k_stage2. */
+ * in shared memory).  Same order of additions as k_stage2.  An addition takes a 16-bit operand
+ * as it is; the instructions beside it bound the kernel (2.6 an addition, with 3 warps a scheduler),
+ * so a DM's offset is one of bytes, that one addition brings to the loads' common base, and the odd
+ * copies are made from 16-byte words: 823 -> 788 us for 5000 DMs of 128 subbands x 13156
+ * samples (bfloat16, 4096 channels), 598 -> 515 for 64 subbands of 1024 channels (float16). */
 template <typename T, int KPC, int TH, int UP>
 __global__ void __launch_bounds__(TH)
 k_stage2p(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long nout,
@@ -870,12 +879,12 @@ k_stage2p(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long no
             }
         }
         __syncthreads();
-        /* word offsets of each (subband, DM): even or odd copy by the parity */
+        /* byte offsets of each (subband, DM): even or odd copy by the parity */
         for (int e = tid; e < sn * KPC; e += TH) {
             const int ss = e / KPC, k = e % KPC;
             const int lo = d2[(size_t)k0 * nsub + s0 + ss];
             const int h = wpos[ss] + wal[ss] + d2[(size_t)(k0 + (k < kn ? k : kn - 1)) * nsub + s0 + ss] - lo;
-            doff[e] = (h & 1) ? (int)(ewords + (h - 1) / 2) : h / 2;
+            doff[e] = 4 * ((h & 1) ? (int)ewords + h / 2 : h / 2);
         }
         for (int ss = tid; ss < sn; ss += TH) {
             const T *row = ring + ((size_t)g * nsub + s0 + ss) * R;
@@ -899,7 +908,7 @@ k_stage2p(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long no
             build_odd(words, ow, nw, tid, TH);
         }
         __syncthreads();
-        const uint32_t *wr = words + tid;
+        const unsigned char *wr = smraw + 4 * tid;
         for (int ss = 0; ss < sn; ss++) {
             const int4 *dv = reinterpret_cast<const int4 *>(doff + ss * KPC);
             int dd[KPC];
@@ -914,7 +923,9 @@ k_stage2p(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long no
 #pragma unroll
             for (int k = 0; k < KPC; k++)
 #pragma unroll
-                for (int q = 0; q < UP; q++) addp(acc[k][2 * q], acc[k][2 * q + 1], wr[dd[k] + q * TH], T());
+                for (int q = 0; q < UP; q++) 
+                    addp(acc[k][2 * q], acc[k][2 * q + 1],
+                         *reinterpret_cast<const uint32_t *>(wr + dd[k] + 4 * q * TH), T());
         }
         __syncthreads();
     }
@@ -1107,16 +1118,42 @@ void launch_stage1(const float *xh, long ldh, long col0, int C, long N, int nsub
 
 
 /* DMs per stage-2 CTA for a group of G fine DMs (one chunk per group when G <= 32). */
-static int stage2_kpc(int G) { return G <= 8 ? 8 : G <= 16 ? 16 : G <= 24 ? 24 : 32; }
+constexpr int S2_MAXK = 32; /* most DMs a stage-2 CTA sums */
 
-/* Largest d2 spread inside one stage-2 DM chunk, over all chunks and subbands. */
+/* DMs a stage-2 CTA sums: a whole group of up to 16, else the part of a group that leaves the
+ * fewest sums over (they are computed and dropped); of equal ones the smallest for FP32, whose time
+ * is the shared-memory reads', and the largest for 16-bit pairs, whose windows are copied twice.
+ * us, this choice (with stage2_kb's windows) against 8, 16, 24 or 32 DMs: 16-bit groups of 40 of
+ * 8192 channels 427 / 726, of 56 1501 / 1885, of 24 of 4096 channels 287 / 348; FP32 groups of
+ * 4 of 256 channels 109 / 168, of 24 of 4096 channels 366 / 406. */
+static int stage2_kpc(int G, bool pairs)
+{
+    if (G <= 16) return (G + 3) / 4 * 4;
+    int best = 0, left = 0;
+    for (int i = 0; i < 6; i++) {
+        const int k = pairs ? 28 - 4 * i : 8 + 4 * i, pad = (G + k - 1) / k * k - G;
+        if (!best || pad < left) best = k, left = pad;
+    }
+    return best;
+}
+
+/* Window budget of a stage-2 CTA in KB: small where few accumulators let many CTAs run on an SM
+ * (one-warp CTAs of 8 DMs, 1024 channels in FP16: 481 us with 12 KB, 516 with 18), large where wide
+ * CTAs share long windows (28 DMs of 8192 channels: 1501 us with 36 KB, 1627 with 18). */
+static int stage2_kb(int k, int G, bool pairs)
+{
+    if (k > 16) return pairs && k == 20 ? 24 : 36;
+    if (pairs) return k <= 12 ? 12 : 18;
+    return k <= 8 && G <= 8 ? 12 : 18;
+}
+
+/* Largest d2 spread inside any S2_MAXK DMs of a group, over all groups and subbands. */
 long stage2_span(const int32_t *d2h, int nsub, int G, long ndm)
 {
-    const long kpc = stage2_kpc(G);
     long span = 0;
     for (long g0 = 0; g0 < ndm; g0 += G)
-        for (long k0 = g0; k0 < min(g0 + (long)G, ndm); k0 += kpc) {
-            long k1 = min(min(k0 + kpc, g0 + (long)G), ndm) - 1;
+        for (long k0 = g0; k0 < min(g0 + (long)G, ndm); k0++) {
+            long k1 = min(min(k0 + S2_MAXK, g0 + (long)G), ndm) - 1;
             for (int s = 0; s < nsub; s++) {
                 long d = (long)d2h[k1 * nsub + s] - d2h[k0 * nsub + s];
                 span = d > span ? d : span;
@@ -1245,9 +1282,10 @@ static void stage2p_impl(const void *ring, long R, int nsub, int G, long ndm, lo
 }
 
 /* FP32 threads per CTA by variant: 0 = 32 (8 samples each; DM chunks wider than 16 take 64),
- * 1 = 64 (4), 2 = 128 (2).  Fewer threads with more samples each load the per-subband delays
- * (broadcast 16-byte loads) for more additions: on the 4096-channel workload variant 0 with
- * 18 KB per CTA took stage 2 from 91 to 81 ms per 20 blocks against 128 threads with 36 KB. */
+ * 1 = 64 (4), 2 = 128 (2; 64 for wider chunks).  Fewer threads with more samples each load the
+ * per-subband delays (broadcast 16-byte loads) for more additions: on the 4096-channel workload
+ * variant 0 with 18 KB per CTA took stage 2 from 91 to 81 ms per 20 blocks against 128 threads
+ * with 36 KB. */
 template <typename T, int K>
 static void stage2_var(int var, const void *ring, long R, int nsub, int G, long ndm, long nout,
                        const int32_t *d2, long span, long t0_mod, float *tim, long ldt, size_t budget,
@@ -1259,15 +1297,18 @@ static void stage2_var(int var, const void *ring, long R, int nsub, int G, long 
             return;
         }
     }
-    if (var == 2)
-        stage2_impl<T, K, 128>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
-    else
-        stage2_impl<T, K, 64>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
+    if constexpr (K <= 16) {
+        if (var == 2) {
+            stage2_impl<T, K, 128>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
+            return;
+        }
+    }
+    stage2_impl<T, K, 64>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
 }
 
 /* 16-bit pair kernel by variant: 0 = 32 threads of 4 pairs (DM chunks wider than 16: 64 of
- * 2), 1 = 64 of 2, 2 = 128 of 1 (variant 0 with 18 KB per CTA: 71 -> 65 ms per 20 blocks of
- * the 4096-channel workload against variant 2 with 36 KB). */
+ * 2), 1 = 64 of 2, 2 = 128 of 1 (64 of 2 for wider chunks).  Variant 0 with 18 KB per CTA:
+ * 71 -> 65 ms per 20 blocks of the 4096-channel workload against variant 2 with 36 KB. */
 template <typename T, int K>
 static void stage2p_var(int var, const void *ring, long R, int nsub, int G, long ndm, long nout,
                         const int32_t *d2, long span, long t0_mod, float *tim, long ldt, size_t budget,
@@ -1279,32 +1320,40 @@ static void stage2p_var(int var, const void *ring, long R, int nsub, int G, long
             return;
         }
     }
-    if (var == 2)
-        stage2p_impl<T, K, 128>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
-    else
-        stage2p_impl<T, K, 64>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
+    if constexpr (K <= 16) {
+        if (var == 2) {
+            stage2p_impl<T, K, 128>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
+            return;
+        }
+    }
+    stage2p_impl<T, K, 64>(ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st);
 }
 
 template <typename T, bool PAIRS>
 static void stage2_dispatch(int var, const void *ring, long R, int nsub, int G, long ndm, long nout,
                             const int32_t *d2, long span, long t0_mod, float *tim, long ldt,
-                            size_t budget, int *err, cudaStream_t st)
+                            int kb, int *err, cudaStream_t st)
 {
-    /* variants 3-5: the thread shapes of 0-2 with half the DMs of a group per CTA (8 for
-     * groups up to 24, 16 for 32): half the accumulators, so more CTAs per SM, each subband
-     * window loaded by twice as many CTAs; every DM's sum is the same */
-    const int kfull = stage2_kpc(G);
-    const int kuse = var >= 3 ? (kfull == 32 ? 16 : 8) : kfull;
+    /* variants 3-5: the thread shapes of 0-2 with at most 8 DMs per CTA: fewer accumulators, so
+     * more CTAs per SM, each subband window loaded by more CTAs; every DM's sum is the same */
+    const int kfull = stage2_kpc(G, PAIRS);
+    int kuse = var >= 3 ? std::min(kfull, 8) : kfull;
+    if ((ndm + G - 1) / G * ((G + kuse - 1) / kuse) > 65535 && G > 16) kuse = S2_MAXK; /* the grid's y */
     const int v = var >= 3 ? var - 3 : var;
+    const size_t budget = (size_t)(kb >= 8 ? kb : stage2_kb(kuse, G, PAIRS)) * 1024;
 #define TXG_S2(K)                                                                                   \
     if constexpr (PAIRS)                                                                            \
         stage2p_var<T, K>(v, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st); \
     else                                                                                            \
         stage2_var<T, K>(v, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget, err, st)
     switch (kuse) {
+    case 4: TXG_S2(4); break;
     case 8: TXG_S2(8); break;
+    case 12: TXG_S2(12); break;
     case 16: TXG_S2(16); break;
+    case 20: TXG_S2(20); break;
     case 24: TXG_S2(24); break;
+    case 28: TXG_S2(28); break;
     default: TXG_S2(32); break;
     }
 #undef TXG_S2
@@ -1344,16 +1393,14 @@ void launch_stage2(const void *ring, long R, int nsub, int G, long ndm, long nou
                    const int32_t *d2, long span, long t0_mod, int prec, int s2_var, int s2_kb,
                    float *tim, long ldt, int *err, cudaStream_t st)
 {
-    /* s2_kb 0: 18 KB per CTA (one-warp CTAs, about twelve per SM) */
-    const size_t budget = (size_t)(s2_kb >= 8 ? s2_kb : 18) * 1024;
     if (prec == TXG_PREC_BF16)
         stage2_dispatch<__nv_bfloat16, true>(s2_var, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt,
-                                             budget, err, st);
+                                             s2_kb, err, st);
     else if (prec == TXG_PREC_FP16)
-        stage2_dispatch<__half, true>(s2_var, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget,
+        stage2_dispatch<__half, true>(s2_var, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, s2_kb,
                                       err, st);
     else
-        stage2_dispatch<float, false>(s2_var, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, budget,
+        stage2_dispatch<float, false>(s2_var, ring, R, nsub, G, ndm, nout, d2, span, t0_mod, tim, ldt, s2_kb,
                                       err, st);
 }
 

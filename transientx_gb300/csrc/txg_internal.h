@@ -159,7 +159,7 @@ void launch_stage1(const float *xh, long ldh, long col0, int C, long N, int nsub
                    cudaStream_t st);
 long stage2_span(const int32_t *d2h, int nsub, int G, long ndm);
 long stage2_window(long span);
-/* s2_var: threads per CTA (0 = 32, 1 = 64, 2 = 128; 3-5 the same with half a group's DMs per
+/* s2_var: threads per CTA (0 = 32, 1 = 64, 2 = 128; 3-5 the same with at most 8 DMs per
  * CTA); s2_kb: shared-memory budget of one stage-2 CTA in KB, 0 = the kernel's default (CTAs
  * per SM follow from it) */
 void launch_stage2(const void *ring, long R, int nsub, int G, long ndm, long nout,
