@@ -131,8 +131,8 @@ void launch_kadaneT(float *x, long ldx, int C, long N, int tdk, int fdk, float t
                     long bwlimit, float *ds, int32_t *ranges, bool have_ds, cudaStream_t st);
 /* mask: pixels of the td x fd downsampled block outside [Q1 - t*R, Q3 + t*R] are zapped;
  * sel: device scratch of MASK_SEL_WORDS words (selection state, then Q1, Q3 and the two
- * limits as float bits); nzap: device int receiving the number of zapped pixels. */
-constexpr int MASK_SEL_WORDS = 2 * 256 + 8;
+ * limits as float bits, a count of CTAs); nzap: device int receiving the number of zapped pixels. */
+constexpr int MASK_SEL_WORDS = 2 * 256 + 9;
 void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr, float *ds,
                  uint32_t *sel, int32_t *nzap, bool have_ds, cudaStream_t st);
 /* zp: C (mean, 1/sd) pairs of scratch */

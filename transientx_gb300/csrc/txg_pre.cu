@@ -370,17 +370,37 @@ __global__ void __launch_bounds__(256) k_unpack(const uint8_t *__restrict__ raw,
     }
 }
 
-/* Unpack for fd | 16 and 16-byte rows: each thread sums, for one output sample, the td raw
- * rows of one 16-channel group (one 16-byte load per row; 16/fd output channels), and a
- * shared-memory transpose gives channel-major coalesced writes.  The sums are of integers
- * below 2^24, exact in FP32, so they equal k_unpack's in any order.
+/* Unpack for fd | 16 and rows of whole words (W: 16-byte rows one load, 4-byte rows four): each
+ * thread sums, for one output sample, the td raw rows of one 16-channel group (16/fd output
+ * channels), and a shared-memory transpose gives channel-major coalesced writes.  The sums are of
+ * integers below 2^24, exact in FP32, so they equal k_unpack's in any order.
  * With `part`, the CTA also writes, per output channel, the exact integer sums of its 64
  * values and of their squares (part[(j*gridDim.x + tile)*2 + {0,1}]): equalize's statistics
- * without another pass over the block. */
+ * without another pass over the block.
+ * SMALL (td * fd <= UV_SMALL: a tile's sum of squares stays below 2^32): two bytes a word are
+ * summed as 16-bit lanes, statistics are 32-bit, and the float is made from the integer's bits; the
+ * conversions (a quarter-rate instruction per byte, then per value and back) bounded the kernel.
+ * 4096 channels x 13156 samples (beside other rows' kernels) 60 -> 53 us, 8192 x 62496 350 -> 316. */
 constexpr int UV_BYTES = 128;  /* raw bytes (channels) per CTA row: 8 groups of 16 */
 constexpr int UV_TI = 64;      /* output samples per CTA */
 
-template <int FD>
+constexpr int UV_SMALL = 40;
+
+template <typename W> __device__ __forceinline__ void uv_load(uint32_t (&w)[4], const uint8_t *p, int left)
+{
+    if constexpr (sizeof(W) == 16) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(p);
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = 4 * k < left ? reinterpret_cast<const uint32_t *>(p)[k] : 0u;
+    }
+}
+
+template <int FD, typename W, bool SMALL>
 __global__ void __launch_bounds__(256) k_unpack_vec(const uint8_t *__restrict__ raw, int C_raw,
                                                    long n0, int td, float *__restrict__ x, long ldx,
                                                    int C, long N, const uint8_t *__restrict__ mask,
@@ -388,36 +408,60 @@ __global__ void __launch_bounds__(256) k_unpack_vec(const uint8_t *__restrict__ 
 {
     constexpr int TJ = UV_BYTES / FD; /* output channels per CTA */
     constexpr int PER = 16 / FD;      /* output channels per thread */
-    __shared__ float outt[TJ][UV_TI + 1];
+    __shared__ uint32_t outt[TJ][UV_TI + 1]; /* integers (SMALL), or floats' bits */
     const int q = threadIdx.x & 7, srow = threadIdx.x >> 3; /* 16-byte group, sample slot 0..31 */
     const int c0 = blockIdx.y * UV_BYTES + 16 * q;         /* first raw channel of the group */
     const long i0 = (long)blockIdx.x * UV_TI;
-    uint4 mk = make_uint4(0u, 0u, 0u, 0u);
     const bool in_c = c0 < C_raw;
-    if (mask && in_c) mk = *reinterpret_cast<const uint4 *>(mask + c0);
-    const uint32_t mw[4] = {mk.x, mk.y, mk.z, mk.w};
+    uint32_t keep[4] = {~0u, ~0u, ~0u, ~0u}; /* bytes of the channels that stay */
+    if (mask && in_c) {
+        uint32_t mw[4];
+        uv_load<W>(mw, mask + c0, C_raw - c0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) keep[k] = __vcmpeq4(mw[k], 0u);
+    }
 #pragma unroll
     for (int pass = 0; pass < UV_TI / 32; pass++) {
         const int ii = pass * 32 + srow;
         const long i = i0 + ii;
-        float acc[PER];
+        const bool in = in_c && i < N;
+        const uint8_t *src = raw + (i * td) * (long)C_raw + c0;
+        if constexpr (SMALL) {
+            uint32_t lo[4] = {0u, 0u, 0u, 0u}, hi[4] = {0u, 0u, 0u, 0u}, acc[PER];
+            if (in) {
+                for (int t = 0; t < td; t++) {
+                    uint32_t w[4];
+                    uv_load<W>(w, src + (long)t * C_raw, C_raw - c0);
 #pragma unroll
-        for (int o = 0; o < PER; o++) acc[o] = 0.f;
-        if (in_c && i < N) {
-            const uint8_t *src = raw + (i * td) * (long)C_raw + c0;
-            for (int t = 0; t < td; t++) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(src + (long)t * C_raw);
-                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int b = 0; b < 16; b++) {
-                    const uint32_t byte = (w[b >> 2] >> (8 * (b & 3))) & 255u;
-                    const uint32_t m = (mw[b >> 2] >> (8 * (b & 3))) & 255u;
-                    acc[b / FD] = __fadd_rn(acc[b / FD], m ? 0.f : (float)byte);
+                    for (int k = 0; k < 4; k++) {
+                        lo[k] += w[k] & keep[k] & 0x00ff00ffu;
+                        hi[k] += (w[k] & keep[k]) >> 8 & 0x00ff00ffu;
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int o = 0; o < PER; o++) outt[q * PER + o][ii] = acc[o];
+            for (int o = 0; o < PER; o++) acc[o] = 0u;
+#pragma unroll
+            for (int b = 0; b < 16; b++)
+                acc[b / FD] += (((b & 1) ? hi[b >> 2] : lo[b >> 2]) >> (8 * (b & 2))) & 0xffffu;
+#pragma unroll
+            for (int o = 0; o < PER; o++) outt[q * PER + o][ii] = acc[o];
+        } else {
+            float acc[PER];
+#pragma unroll
+            for (int o = 0; o < PER; o++) acc[o] = 0.f;
+            if (in) {
+                for (int t = 0; t < td; t++) {
+                    uint32_t w[4];
+                    uv_load<W>(w, src + (long)t * C_raw, C_raw - c0);
+#pragma unroll
+                    for (int b = 0; b < 16; b++)
+                        acc[b / FD] = __fadd_rn(acc[b / FD], (float)(((w[b >> 2] & keep[b >> 2]) >> (8 * (b & 3))) & 255u));
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < PER; o++) outt[q * PER + o][ii] = __float_as_uint(acc[o]);
+        }
     }
     __syncthreads();
     const int j0 = blockIdx.y * TJ;
@@ -425,7 +469,10 @@ __global__ void __launch_bounds__(256) k_unpack_vec(const uint8_t *__restrict__ 
         const int jj = e / UV_TI, ii = e % UV_TI;
         const int j = j0 + jj;
         const long i = i0 + ii;
-        if (j < C && i < N) x[(long)j * ldx + i] = outt[jj][ii];
+        const uint32_t v = outt[jj][ii];
+        /* v < 2^23: 2^23 + v as bits, less 2^23 */
+        const float f = SMALL ? __fsub_rn(__uint_as_float(0x4b000000u | v), 8388608.f) : __uint_as_float(v);
+        if (j < C && i < N) x[(long)j * ldx + i] = f;
     }
     if (part) {
         /* samples past N hold 0 and add nothing; values are exact non-negative integers */
@@ -433,11 +480,24 @@ __global__ void __launch_bounds__(256) k_unpack_vec(const uint8_t *__restrict__ 
         __shared__ unsigned long long ps[TPC > 1 ? TPC - 1 : 1][TJ][2];
         const int jj = threadIdx.x % TJ, pt = threadIdx.x / TJ;
         unsigned long long a1 = 0ull, a2 = 0ull;
+        if constexpr (SMALL) {
+            static_assert((uint64_t)UV_TI * (255 * UV_SMALL) * (255 * UV_SMALL) / 2 < 1ull << 32, "squares in 32 bits");
+            uint32_t b1 = 0u, b2 = 0u;
 #pragma unroll 8
-        for (int k = 0; k < SPT; k++) {
-            const unsigned v = __float2uint_rz(outt[jj][pt * SPT + k]);
-            a1 += v;
-            a2 += (unsigned long long)v * v;
+            for (int k = 0; k < SPT; k++) {
+                const uint32_t v = outt[jj][pt * SPT + k];
+                b1 += v;
+                b2 += v * v;
+            }
+            a1 = b1;
+            a2 = b2;
+        } else {
+#pragma unroll 8
+            for (int k = 0; k < SPT; k++) {
+                const unsigned v = __float2uint_rz(__uint_as_float(outt[jj][pt * SPT + k]));
+                a1 += v;
+                a2 += (unsigned long long)v * v;
+            }
         }
         if (pt > 0) {
             ps[pt - 1][jj][0] = a1;
@@ -964,8 +1024,9 @@ __global__ void k_kadaneT_apply(float *__restrict__ x, long ldx, long N, int tdk
 /* ---- mask ------------------------------------------------------------------------------- */
 /* Exact order statistics of the downsampled block by radix selection on order-preserving
  * 32-bit keys: four 8-bit passes, each a histogram of the keys that still match the selected
- * prefix (two targets at once, Q1 and Q3) and a one-thread pick of the digit holding the
- * remaining rank.  sel: [0,512) histograms, 512.. prefix/rank per target, 516.. results. */
+ * prefix (two targets at once, Q1 and Q3) whose last CTA picks the digit holding the
+ * remaining rank.  sel: [0,512) histograms, 512.. prefix/rank per target, 516.. results, 520 the
+ * CTAs that are done. */
 __device__ __forceinline__ uint32_t order_key(float f)
 {
     const uint32_t u = __float_as_uint(f);
@@ -976,10 +1037,14 @@ __device__ __forceinline__ float order_key_inv(uint32_t k)
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+__device__ void mask_pick(uint32_t *__restrict__ sel, int shift, uint32_t k0, uint32_t k1, float thr);
+
 __global__ void __launch_bounds__(256) k_mask_hist(const float *__restrict__ ds, long n,
-                                                   uint32_t *__restrict__ sel, int shift)
+                                                   uint32_t *__restrict__ sel, int shift, uint32_t k0,
+                                                   uint32_t k1, float thr)
 {
     __shared__ uint32_t h[512];
+    __shared__ bool last;
     for (int b = threadIdx.x; b < 512; b += blockDim.x) h[b] = 0;
     __syncthreads();
     const uint32_t p0 = sel[512], p1 = sel[514];
@@ -993,29 +1058,60 @@ __global__ void __launch_bounds__(256) k_mask_hist(const float *__restrict__ ds,
     __syncthreads();
     for (int b = threadIdx.x; b < 512; b += blockDim.x)
         if (h[b]) atomicAdd(&sel[b], h[b]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&sel[520], 1u) + 1 == gridDim.x;
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        mask_pick(sel, shift, k0, k1, thr);
+    }
 }
 
-__global__ void k_mask_pick(uint32_t *__restrict__ sel, int shift, uint32_t k0, uint32_t k1,
-                            float thr)
+/* The digit of each target's rank, by the histogram's last CTA: warp t takes target t, eight bins a
+ * lane.  (One thread of a kernel of its own walked the bins before: 8 to 16 us a digit, beside 3 to
+ * 5 for the histogram; the two in one take 5.) */
+__device__ void mask_pick(uint32_t *__restrict__ sel, int shift, uint32_t k0, uint32_t k1, float thr)
 {
-    if (threadIdx.x != 0) return;
-    for (int t = 0; t < 2; t++) {
-        uint32_t prefix = shift == 24 ? 0u : sel[512 + 2 * t];
-        uint32_t rank = shift == 24 ? (t == 0 ? k0 : k1) : sel[513 + 2 * t];
-        uint32_t cum = 0, digit = 255;
-        for (uint32_t b = 0; b < 256; b++) {
-            const uint32_t c = sel[256 * t + b];
-            if (rank < cum + c) {
-                digit = b;
-                break;
-            }
-            cum += c;
+    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (t < 2) {
+        const uint32_t prefix = shift == 24 ? 0u : __ldcg(sel + 512 + 2 * t);
+        const uint32_t rank = shift == 24 ? (t == 0 ? k0 : k1) : __ldcg(sel + 513 + 2 * t);
+        uint32_t c[8], sum = 0;
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+            c[b] = __ldcg(sel + 256 * t + 8 * lane + b);
+            sum += c[b];
         }
-        sel[512 + 2 * t] = prefix | (digit << shift);
-        sel[513 + 2 * t] = rank - cum;
+        uint32_t cum = sum; /* counts up to this lane's last bin */
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, cum, off);
+            if (lane >= off) cum += y;
+        }
+        const uint32_t all = __shfl_sync(FULL, cum, 31);
+        const unsigned hit = __ballot_sync(FULL, rank < cum);
+        if (hit == 0) { /* beyond the last: the last digit */
+            if (lane == 0) {
+                sel[512 + 2 * t] = prefix | (255u << shift);
+                sel[513 + 2 * t] = rank - all;
+            }
+        } else if (lane == __ffs(hit) - 1) {
+            uint32_t before = cum - sum, digit = 8 * lane;
+            for (int b = 0; b < 8; b++) {
+                if (rank < before + c[b]) break;
+                before += c[b];
+                digit++;
+            }
+            sel[512 + 2 * t] = prefix | (digit << shift);
+            sel[513 + 2 * t] = rank - before;
+        }
+#pragma unroll
+        for (int b = 0; b < 8; b++) sel[256 * t + 8 * lane + b] = 0;
     }
-    for (int b = 0; b < 512; b++) sel[b] = 0;
-    if (shift == 0) {
+    __syncthreads();
+    if (threadIdx.x == 0) sel[520] = 0;
+    if (shift == 0 && threadIdx.x == 0) {
         const float q1 = order_key_inv(sel[512]), q3 = order_key_inv(sel[514]);
         const float r = __fsub_rn(q3, q1);
         const float lo = __fsub_rn(q1, __fmul_rn(thr, r)), hi = __fadd_rn(q3, __fmul_rn(thr, r));
@@ -1177,21 +1273,37 @@ void launch_skzap(const uint8_t *raw, int C_raw, long n0, float thr, unsigned lo
 
 long eq_part_tiles(long N) { return (long)nblk(N, UV_TI); }
 
+template <int FD, typename W>
+static void unpack_vec(dim3 grid, const uint8_t *raw, int C_raw, long n0, int td, float *x, long ldx, int C, long N,
+                       const uint8_t *mask, unsigned long long *part, cudaStream_t st)
+{
+    if (td <= UV_SMALL / FD)
+        k_unpack_vec<FD, W, true><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part);
+    else
+        k_unpack_vec<FD, W, false><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part);
+}
+
 bool launch_unpack(const uint8_t *raw, int C_raw, long n0, int td, int fd, float *x, long ldx,
                    int C, long N, const uint8_t *mask, unsigned long long *part, cudaStream_t st)
 {
-    const bool vec = C_raw % 16 == 0 && (reinterpret_cast<uintptr_t>(raw) & 15) == 0 &&
-                     (!mask || (reinterpret_cast<uintptr_t>(mask) & 15) == 0) &&
-                     (fd == 1 || fd == 2 || fd == 4 || fd == 8 || fd == 16);
-    if (vec) {
+    /* rows of whole words; 1000 channels x 4995 samples folded by 2 took k_unpack 48 us and k_eq_params,
+     * without these sums, 18; now 8 and 6.  Other rows and folds keep k_unpack. */
+    const uintptr_t al = reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(mask) | (uintptr_t)C_raw;
+    if ((al & 3) == 0 && (fd == 1 || fd == 2 || fd == 4 || fd == 8 || fd == 16)) {
         dim3 grid(nblk(N, UV_TI), nblk(C_raw, UV_BYTES));
+#define TXG_UV(FD)                                                                                     \
+    if ((al & 15) == 0)                                                                                \
+        unpack_vec<FD, uint4>(grid, raw, C_raw, n0, td, x, ldx, C, N, mask, part, st);                 \
+    else                                                                                               \
+        unpack_vec<FD, uint32_t>(grid, raw, C_raw, n0, td, x, ldx, C, N, mask, part, st)
         switch (fd) {
-        case 1: k_unpack_vec<1><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part); break;
-        case 2: k_unpack_vec<2><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part); break;
-        case 4: k_unpack_vec<4><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part); break;
-        case 8: k_unpack_vec<8><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part); break;
-        default: k_unpack_vec<16><<<grid, 256, 0, st>>>(raw, C_raw, n0, td, x, ldx, C, N, mask, part); break;
+        case 1: TXG_UV(1); break;
+        case 2: TXG_UV(2); break;
+        case 4: TXG_UV(4); break;
+        case 8: TXG_UV(8); break;
+        default: TXG_UV(16); break;
         }
+#undef TXG_UV
         return part != nullptr;
     }
     size_t smem = (size_t)UP_TI * td * UP_TJ * fd;
@@ -1339,10 +1451,7 @@ void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
     /* ranks of the quartiles, as the channel zap takes them: sorted[n/4], sorted[n-1-n/4] */
     const uint32_t k0 = (uint32_t)(n / 4), k1 = (uint32_t)(n - 1 - n / 4);
     const unsigned hb = (unsigned)std::min<long>(nblk(n, 256), 152L * 8);
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        k_mask_hist<<<hb, 256, 0, st>>>(ds, n, sel, shift);
-        k_mask_pick<<<1, 32, 0, st>>>(sel, shift, k0, k1, thr);
-    }
+    for (int shift = 24; shift >= 0; shift -= 8) k_mask_hist<<<hb, 256, 0, st>>>(ds, n, sel, shift, k0, k1, thr);
     dim3 g3(nblk(N, 256), Cds * fdk);
     k_mask_apply<<<g3, 256, 0, st>>>(x, ldx, N, Cds, Nds, tdk, fdk, ds, sel, nzap);
 }
