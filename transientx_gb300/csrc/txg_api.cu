@@ -572,6 +572,7 @@ int run_block(txg_handle *h, int beam, const uint8_t *raw, const float *rawf = n
         TXG_CUDA_TRY(cudaStreamWaitEvent(rs, h->fork, 0));
         if (timing) TXG_CUDA_TRY(cudaEventRecord(sl.ev[0], rs));
 
+        TXG_CUDA_TRY(cudaMemsetAsync(sl.dcount, 0, 2 * sizeof(int), rs));
         /* history: the last H columns of the previous block go in front of this one */
         /* one buffer when the history is shorter than a block (the previous block's last H
          * columns [N, N+H) move to [0, H), stream-ordered after its stage 1); two otherwise */
@@ -633,7 +634,6 @@ int run_block(txg_handle *h, int beam, const uint8_t *raw, const float *rawf = n
         /* stage 1: new subband samples t in [counter-N-maxd1, counter-maxd1) */
         const long counter = b.pushed + P.N;
         const long tbase = counter - P.N - P.maxd1;
-        TXG_CUDA_TRY(cudaMemsetAsync(sl.dcount, 0, 2 * sizeof(int), rs));
         launch_stage1(xcur, P.ldh, P.H - P.maxd1, P.C, P.N, P.nsub, P.ng, D.sub_start, D.d1,
                       P.maxd1, P.maxch, b.ring, P.R, pmod(tbase, P.R), h->prec, P.s1_var, D.s1t,
                       sl.dcount + 1, rs);

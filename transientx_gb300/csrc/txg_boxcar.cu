@@ -589,6 +589,7 @@ k_boxcar(const float *__restrict__ tim, long ldt, long n, const int32_t *__restr
          int nw, int iqr, float thre, txg_cand *__restrict__ cand,
          int *__restrict__ ncand, long cap, float *__restrict__ mxS, int32_t *__restrict__ mxwn)
 {
+    chain_wait();
     extern __shared__ __align__(16) float c[];
     __shared__ double red[2 * BX_THREADS / 32];
     __shared__ float2 mv;
@@ -670,6 +671,7 @@ static int prep_chunks(long L)
 __global__ void __launch_bounds__(BX_THREADS)
 k_boxcar_prep(const float *__restrict__ tim, long ldt, long n, int iqr, int pc, double *__restrict__ scratch)
 {
+    chain_wait();
     extern __shared__ __align__(16) float c[];
     __shared__ double red[2 * BX_THREADS / 32];
     __shared__ float2 mv;
@@ -717,6 +719,7 @@ k_boxcar_seg(const float *__restrict__ tim, long ldt, long n, const int32_t *__r
              int nw, float thre, const double *__restrict__ scratch, txg_cand *__restrict__ cand,
              int *__restrict__ ncand, long cap, float *__restrict__ mxS, int32_t *__restrict__ mxwn)
 {
+    chain_wait();
     extern __shared__ __align__(16) float c[];
     __shared__ float temp_w[256];
     __shared__ int4 wpar[256];
@@ -824,8 +827,8 @@ int launch_boxcar(const float *tim, long ldt, long ndm, long n, const int32_t *v
 #define TXG_BX(A, T, B)                                                                               \
     do {                                                                                              \
         cudaFuncSetAttribute(k_boxcar<A, T, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BX_SMEM_TOP); \
-        k_boxcar<A, T, B><<<(unsigned)ndm, BX_THREADS, smem, st>>>(tim, ldt, n, vwn, nw, iqr, thre, cand, ncand, \
-                                                                    cap, mxS, mxwn);                   \
+        launch_chained(k_boxcar<A, T, B>, (unsigned)ndm, BX_THREADS, smem, st, tim, ldt, n, vwn, nw, iqr, thre, \
+                       cand, ncand, cap, mxS, mxwn);                                                  \
     } while (0)
         if (avx2_tail)
             TXG_BX(true, true, false);
@@ -849,13 +852,13 @@ int launch_boxcar(const float *tim, long ldt, long ndm, long n, const int32_t *v
     const size_t smem = boxcar_smem(nc, bound), psmem = (size_t)(BX_THREADS / 32) * prep_chunks(L) * L * sizeof(float);
     if (smem > BX_SMEM_TOP || psmem > BX_SMEM_TOP) return TXG_ERR_UNSUPPORTED;
     cudaFuncSetAttribute(k_boxcar_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
-    k_boxcar_prep<<<(unsigned)ndm, BX_THREADS, psmem, st>>>(tim, ldt, n, iqr, prep_chunks(L), scratch);
+    launch_chained(k_boxcar_prep, (unsigned)ndm, BX_THREADS, psmem, st, tim, ldt, n, iqr, prep_chunks(L), scratch);
     dim3 grid((unsigned)ndm, (unsigned)nseg);
 #define TXG_BXS(A, T, B)                                                                              \
     do {                                                                                              \
         cudaFuncSetAttribute(k_boxcar_seg<A, T, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        k_boxcar_seg<A, T, B><<<grid, BX_THREADS, smem, st>>>(tim, ldt, n, vwn, nw, thre, scratch, cand, ncand, \
-                                                               cap, mxS, mxwn);                        \
+        launch_chained(k_boxcar_seg<A, T, B>, grid, BX_THREADS, smem, st, tim, ldt, n, vwn, nw, thre, scratch, \
+                       cand, ncand, cap, mxS, mxwn);                                                  \
     } while (0)
     if (avx2_tail)
         TXG_BXS(true, true, false);

@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "txg_device.cuh"
 #include "txg_internal.h"
 
 namespace txg {
@@ -469,6 +470,7 @@ k_stage1t(const float *__restrict__ xh, long ldh, long col0, int C, long N, int 
           const int32_t *__restrict__ first, int npass, int qpt, int cw, int nb,
           const int32_t *__restrict__ span, int maxch, T *__restrict__ ring, long R, long tbase_mod)
 {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ uint32_t tm_slot;
     /* the shuffle tells the compiler that all of a warp has the same wp */
@@ -673,6 +675,7 @@ k_stage2(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long nou
          const int32_t *__restrict__ d2, long t0_mod, int sc, long wtot_max,
          float *__restrict__ tim, long ldt, int *err)
 {
+    chain_wait();
     static_assert(TH * U == S2_TT && TH >= 32, "the tile is S2_TT samples");
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ __align__(8) uint64_t bar;
@@ -810,6 +813,7 @@ k_stage2p(const T *__restrict__ ring, long R, int nsub, int G, long ndm, long no
           const int32_t *__restrict__ d2, long t0_mod, int sc, long wtot_max,
           float *__restrict__ tim, long ldt, int *err)
 {
+    chain_wait();
     constexpr int TT = 2 * TH * UP;
     static_assert(TT == S2_TT && TH >= 32, "the tile is S2_TT samples");
     constexpr int EPC = 8; /* 16-bit elements per 16 bytes */
@@ -1040,9 +1044,8 @@ static void stage1t(const Stage1TDev &t, const float *xh, long ldh, long col0, i
     const size_t smem = stage1t_smem(maxch, t.npass, t.widest);
     auto kern = k_stage1t<T>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<dim3(nblk(N + (tbase_mod & 15), S1T_TT), nsub), S1T_THREADS, smem, st>>>(
-        xh, ldh, col0, C, N, nsub, ng, sub_start, t.rel, t.first, t.npass, t.qpt, t.cw, t.nb, t.span, maxch,
-        ring, R, tbase_mod);
+    launch_chained(kern, dim3(nblk(N + (tbase_mod & 15), S1T_TT), nsub), S1T_THREADS, smem, st, xh, ldh, col0, C, N,
+                   nsub, ng, sub_start, t.rel, t.first, t.npass, t.qpt, t.cw, t.nb, t.span, maxch, ring, R, tbase_mod);
 }
 
 /* Resident launch shapes (threads per set x samples per thread, thread sets x groups each),
@@ -1252,8 +1255,8 @@ static void stage2_impl(const void *ring, long R, int nsub, int G, long ndm, lon
     dim3 grid(nblk(nout, S2_TT), (unsigned)(ng * nkc));
     auto kern = k_stage2<T, KPC, TH, S2_TT / TH>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<grid, TH, smem, st>>>((const T *)ring, R, nsub, G, ndm, nout, d2, t0_mod, sc, wtot, tim, ldt,
-                                 err);
+    launch_chained(kern, grid, TH, smem, st, (const T *)ring, R, nsub, G, ndm, nout, d2, t0_mod, sc, wtot, tim, ldt,
+                   err);
 }
 
 /* 16-bit ring: pair kernel, TH threads of UP pairs over the S2_TT-sample tile, windows doubled
@@ -1277,8 +1280,8 @@ static void stage2p_impl(const void *ring, long R, int nsub, int G, long ndm, lo
     dim3 grid(nblk(nout, S2_TT), (unsigned)(ng * nkc));
     auto kern = k_stage2p<T, KPC, TH, UP>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<grid, TH, smem, st>>>((const T *)ring, R, nsub, G, ndm, nout, d2, t0_mod, sc, wtot, tim, ldt,
-                                 err);
+    launch_chained(kern, grid, TH, smem, st, (const T *)ring, R, nsub, G, ndm, nout, d2, t0_mod, sc, wtot, tim, ldt,
+                   err);
 }
 
 /* FP32 threads per CTA by variant: 0 = 32 (8 samples each; DM chunks wider than 16 take 64),

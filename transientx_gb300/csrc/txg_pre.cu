@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(32 * SK_SLICES) k_sk_sums(const uint8_t *__res
 __global__ void k_sk_stats(const unsigned long long *__restrict__ sums, int C, long n0,
                            double *__restrict__ stats)
 {
+    chain_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const double n = (double)n0;
@@ -241,6 +242,7 @@ __device__ __forceinline__ double dkey_inv(unsigned long long k)
 __global__ void __launch_bounds__(1024) k_sk_select(int C, float thr, const double *__restrict__ stats,
                                                    uint8_t *__restrict__ mask)
 {
+    chain_wait();
     __shared__ unsigned int hist[4][256];
     __shared__ unsigned long long pref[4];
     __shared__ unsigned int rank[4];
@@ -581,6 +583,7 @@ __global__ void __launch_bounds__(FT_J * 8) k_unpack_f32(const float *__restrict
 __global__ void __launch_bounds__(RB_THREADS) k_eq_params_f32(const float *__restrict__ x, long ldx, long N,
                                                               float2 *__restrict__ eqp, uint8_t *__restrict__ live)
 {
+    chain_wait();
     __shared__ RedRow sh;
     const int c = blockIdx.x;
     const float *r = x + (long)c * ldx;
@@ -607,6 +610,7 @@ __global__ void __launch_bounds__(256) k_eq_params(const unsigned long long *__r
                                                    int C, long N, float2 *__restrict__ eqp,
                                                    uint8_t *__restrict__ live)
 {
+    chain_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= C) return;
     long long s1 = 0, s2 = 0; /* exact integer sums: any order */
@@ -654,6 +658,7 @@ __global__ void __launch_bounds__(256) k_eq_params(const unsigned long long *__r
 __global__ void k_eq_apply(float *__restrict__ x, long ldx, long N, const float2 *__restrict__ eqp,
                            const float *__restrict__ b, const uint8_t *__restrict__ live)
 {
+    chain_wait();
     const long i = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
     const int j = blockIdx.y;
     if (i >= N) return;
@@ -688,6 +693,7 @@ __global__ void __launch_bounds__(256) k_ds(float *__restrict__ x, long ldx, int
                                             const float2 *__restrict__ eqp, const float *__restrict__ b,
                                             const uint8_t *__restrict__ live, float *__restrict__ ds)
 {
+    chain_wait();
     __shared__ float tile[32][33];
     const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const long i = (long)blockIdx.x * 32 + lane, i0 = i * TD;
@@ -751,6 +757,7 @@ __global__ void __launch_bounds__(32 * CSUM_BLK) k_colmean(const float *__restri
                                                          const float2 *__restrict__ tp,
                                                          float *__restrict__ out)
 {
+    chain_wait();
     __shared__ float part[CSUM_BLK][33];
     __shared__ int nlive_sh;
     const int lane = threadIdx.x, q = threadIdx.y;
@@ -802,6 +809,7 @@ constexpr int SM_T = 128, SM_CH = 4096;
 
 __global__ void __launch_bounds__(SM_T) k_smooth(const float *__restrict__ z, long N, long nw, float *__restrict__ b)
 {
+    chain_wait();
     __shared__ float zs[SM_CH];
     const long i0 = (long)blockIdx.x * SM_T, i = i0 + threadIdx.x;
     const long h = nw / 2;
@@ -832,6 +840,7 @@ __global__ void __launch_bounds__(SM_T) k_smooth(const float *__restrict__ z, lo
 __global__ void k_sub_series(float *__restrict__ x, long ldx, long N, const float *__restrict__ b,
                              const uint8_t *__restrict__ live)
 {
+    chain_wait();
     const long i = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
     const int j = blockIdx.y;
     if (i >= N || (live && !live[j])) return;
@@ -852,6 +861,7 @@ __global__ void k_sub_series(float *__restrict__ x, long ldx, long N, const floa
 __global__ void k_zero_rows(float *__restrict__ x, long ldx, const int32_t *__restrict__ rows,
                             long N)
 {
+    chain_wait();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     x[(long)rows[blockIdx.y] * ldx + i] = 0.f;
@@ -862,6 +872,7 @@ __global__ void k_zero_rows(float *__restrict__ x, long ldx, const int32_t *__re
 __global__ void k_kadane_ds(const float *__restrict__ x, long ldx, int Cds, long Nds, int tdk,
                             int fdk, float *__restrict__ ds)
 {
+    chain_wait();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int j = blockIdx.y;
     if (i >= Nds) return;
@@ -896,6 +907,7 @@ __global__ void __launch_bounds__(64) k_kadane_scan(const float *__restrict__ ds
                                                     int tdk, int fdk, float thr, long wnlimit,
                                                     int32_t *__restrict__ ranges)
 {
+    chain_wait();
     __shared__ float tile[KS_NB][KS_T][32];
     const int lane = threadIdx.x & 31, neg = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
     const unsigned flip = neg ? 0x80000000u : 0u;
@@ -955,6 +967,7 @@ __global__ void __launch_bounds__(64) k_kadane_scan(const float *__restrict__ ds
 __global__ void __launch_bounds__(256) k_kadane_apply(float *__restrict__ x, long ldx, long N, int C, int fdk,
                                                       const int32_t *__restrict__ ranges)
 {
+    chain_wait();
     const int jr = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (jr >= C) return;
     const int32_t *r = ranges + 4 * (jr / fdk);
@@ -974,6 +987,7 @@ __global__ void __launch_bounds__(256) k_kadane_apply(float *__restrict__ x, lon
 __global__ void k_kadaneT_scan(const float *__restrict__ ds, int Cds, long Nds, int tdk, int fdk,
                                float thr, long bwlimit, int32_t *__restrict__ ranges)
 {
+    chain_wait();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= Nds) return;
     const float *row = ds + i * Cds;
@@ -1013,6 +1027,7 @@ __global__ void k_kadaneT_scan(const float *__restrict__ ds, int Cds, long Nds, 
 __global__ void k_kadaneT_apply(float *__restrict__ x, long ldx, long N, int tdk, long Nds,
                                 const int32_t *__restrict__ ranges)
 {
+    chain_wait();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int c = blockIdx.y;
     if (t >= N || t / tdk >= Nds) return;
@@ -1043,6 +1058,7 @@ __global__ void __launch_bounds__(256) k_mask_hist(const float *__restrict__ ds,
                                                    uint32_t *__restrict__ sel, int shift, uint32_t k0,
                                                    uint32_t k1, float thr)
 {
+    chain_wait();
     __shared__ uint32_t h[512];
     __shared__ bool last;
     for (int b = threadIdx.x; b < 512; b += blockDim.x) h[b] = 0;
@@ -1126,6 +1142,7 @@ __global__ void k_mask_apply(float *__restrict__ x, long ldx, long N, int Cds, l
                              int fdk, const float *__restrict__ ds, const uint32_t *__restrict__ sel,
                              int32_t *__restrict__ nzap)
 {
+    chain_wait();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int c = blockIdx.y;
     const long i = t / tdk;
@@ -1146,6 +1163,7 @@ __global__ void k_mask_apply(float *__restrict__ x, long ldx, long N, int Cds, l
 __global__ void __launch_bounds__(RB_THREADS) k_zdot_norm(const float *__restrict__ x, long ldx, long N,
                                                           float2 *__restrict__ zp)
 {
+    chain_wait();
     __shared__ RedRow sh;
     const float *r = x + (long)blockIdx.x * ldx;
     double s1, s2;
@@ -1167,6 +1185,7 @@ constexpr int SST_RUNS = 4096; /* run totals staged per lane set (2 floats each)
 __global__ void __launch_bounds__(1024) k_zdot_sstats(const float *__restrict__ s, long N,
                                                      double *__restrict__ out)
 {
+    chain_wait();
     __shared__ float run1[SST_RUNS], run2[SST_RUNS];
     const long nruns = ((N + 31) / 32 + RED_RUN - 1) / RED_RUN; /* runs of the longest lane */
     double a1 = 0., a2 = 0.;
@@ -1218,6 +1237,7 @@ __global__ void __launch_bounds__(RB_THREADS) k_zdot_fit(float *__restrict__ x, 
                                                          const float *__restrict__ s,
                                                          const double *__restrict__ sst)
 {
+    chain_wait();
     extern __shared__ float row[];
     __shared__ RedRow sh;
     __shared__ float2 ab;
@@ -1267,8 +1287,8 @@ void launch_skzap(const uint8_t *raw, int C_raw, long n0, float thr, unsigned lo
     const int vec = (C_raw % 4 == 0) && ((reinterpret_cast<uintptr_t>(raw) & 3) == 0);
     dim3 g1(nblk(C_raw, 128), nblk(n0, SK_TCHUNK));
     k_sk_sums<<<g1, dim3(32, SK_SLICES), 0, st>>>(raw, C_raw, n0, vec, sums);
-    k_sk_stats<<<nblk(C_raw, 256), 256, 0, st>>>(sums, C_raw, n0, stats);
-    k_sk_select<<<1, 1024, 0, st>>>(C_raw, thr, stats, mask);
+    launch_chained(k_sk_stats, nblk(C_raw, 256), 256, 0, st, sums, C_raw, n0, stats);
+    launch_chained(k_sk_select, 1, 1024, 0, st, C_raw, thr, stats, mask);
 }
 
 long eq_part_tiles(long N) { return (long)nblk(N, UV_TI); }
@@ -1324,7 +1344,7 @@ bool launch_unpack(const uint8_t *raw, int C_raw, long n0, int td, int fd, float
 void launch_eq_params(const unsigned long long *part, const float *x, long ldx, int C, long N,
                       float2 *eqp, uint8_t *live, cudaStream_t st)
 {
-    k_eq_params<<<nblk((long)C * 32, 256), 256, 0, st>>>(part, eq_part_tiles(N), x, ldx, C, N, eqp, live);
+    launch_chained(k_eq_params, nblk((long)C * 32, 256), 256, 0, st, part, eq_part_tiles(N), x, ldx, C, N, eqp, live);
 }
 
 void launch_unpack_f32(const float *blk, int C_raw, long n0, int td, int fd, float *x, long ldx,
@@ -1338,7 +1358,7 @@ void launch_unpack_f32(const float *blk, int C_raw, long n0, int td, int fd, flo
 void launch_eq_params_f32(const float *x, long ldx, int C, long N, float2 *eqp, uint8_t *live,
                           cudaStream_t st)
 {
-    k_eq_params_f32<<<C, RB_THREADS, 0, st>>>(x, ldx, N, eqp, live);
+    launch_chained(k_eq_params_f32, C, RB_THREADS, 0, st, x, ldx, N, eqp, live);
 }
 
 /* k_ds where it applies (td 4, 8 or 16 and aligned rows): with eqp also the equalize apply. */
@@ -1355,9 +1375,9 @@ static bool downsample(float *x, long ldx, int C, long N, int td, int fd, const 
 #define TXG_DS(TD)                                                                                     \
     do {                                                                                               \
         if (eqp)                                                                                       \
-            k_ds<TD, true><<<grid, 256, 0, st>>>(x, ldx, C, N, fd, Cds, Nds, eqp, b, live, ds);        \
+            launch_chained(k_ds<TD, true>, grid, 256, 0, st, x, ldx, C, N, fd, Cds, Nds, eqp, b, live, ds);        \
         else                                                                                           \
-            k_ds<TD, false><<<grid, 256, 0, st>>>(x, ldx, C, N, fd, Cds, Nds, nullptr, nullptr, nullptr, ds); \
+            launch_chained(k_ds<TD, false>, grid, 256, 0, st, x, ldx, C, N, fd, Cds, Nds, nullptr, nullptr, nullptr, ds); \
         return true;                                                                                   \
     } while (0)
     if (td == 4) TXG_DS(4);
@@ -1370,7 +1390,7 @@ static bool downsample(float *x, long ldx, int C, long N, int td, int fd, const 
 static void kadane_ds(float *x, long ldx, int Cds, long Nds, int C, long N, int td, int fd, float *ds, cudaStream_t st)
 {
     if (!downsample(x, ldx, C, N, td, fd, nullptr, nullptr, nullptr, ds, st))
-        k_kadane_ds<<<dim3(nblk(Nds, 128), Cds), 128, 0, st>>>(x, ldx, Cds, Nds, td, fd, ds);
+        launch_chained(k_kadane_ds, dim3(nblk(Nds, 128), Cds), 128, 0, st, x, ldx, Cds, Nds, td, fd, ds);
 }
 
 bool launch_eq_apply_ds(float *x, long ldx, int C, long N, const float2 *eqp, const float *b, const uint8_t *live,
@@ -1383,28 +1403,28 @@ void launch_eq_apply(float *x, long ldx, int C, long N, const float2 *eqp, const
                      const uint8_t *live, cudaStream_t st)
 {
     dim3 grid(nblk((N + 3) / 4, 256), C);
-    k_eq_apply<<<grid, 256, 0, st>>>(x, ldx, N, eqp, b, live);
+    launch_chained(k_eq_apply, grid, 256, 0, st, x, ldx, N, eqp, b, live);
 }
 
 void launch_colmean(const float *x, long ldx, int C, long N, const uint8_t *live, const float2 *tp,
                     float *out, cudaStream_t st)
 {
     if (tp)
-        k_colmean<true><<<nblk(N, 32), dim3(32, CSUM_BLK), 0, st>>>(x, ldx, C, N, live, tp, out);
+        launch_chained(k_colmean<true>, nblk(N, 32), dim3(32, CSUM_BLK), 0, st, x, ldx, C, N, live, tp, out);
     else
-        k_colmean<false><<<nblk(N, 32), dim3(32, CSUM_BLK), 0, st>>>(x, ldx, C, N, live, nullptr, out);
+        launch_chained(k_colmean<false>, nblk(N, 32), dim3(32, CSUM_BLK), 0, st, x, ldx, C, N, live, nullptr, out);
 }
 
 void launch_smooth(const float *z, long N, long nw, float *b, cudaStream_t st)
 {
-    k_smooth<<<nblk(N, SM_T), SM_T, 0, st>>>(z, N, nw, b);
+    launch_chained(k_smooth, nblk(N, SM_T), SM_T, 0, st, z, N, nw, b);
 }
 
 void launch_sub_series(float *x, long ldx, int C, long N, const float *b, const uint8_t *live,
                        cudaStream_t st)
 {
     dim3 grid(nblk((N + 3) / 4, 256), C);
-    k_sub_series<<<grid, 256, 0, st>>>(x, ldx, N, b, live);
+    launch_chained(k_sub_series, grid, 256, 0, st, x, ldx, N, b, live);
 }
 
 void launch_zero_rows(float *x, long ldx, const int32_t *rows, int nrows, long N,
@@ -1412,7 +1432,7 @@ void launch_zero_rows(float *x, long ldx, const int32_t *rows, int nrows, long N
 {
     if (nrows <= 0) return;
     dim3 grid(nblk(N, 256), nrows);
-    k_zero_rows<<<grid, 256, 0, st>>>(x, ldx, rows, N);
+    launch_chained(k_zero_rows, grid, 256, 0, st, x, ldx, rows, N);
 }
 
 void launch_kadane(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
@@ -1422,8 +1442,8 @@ void launch_kadane(float *x, long ldx, int C, long N, int tdk, int fdk, float th
     long Nds = N / tdk;
     if (Cds <= 0) return;
     if (Nds > 0 && !have_ds) kadane_ds(x, ldx, Cds, Nds, C, N, tdk, fdk, ds, st);
-    k_kadane_scan<<<nblk(Cds, 32), 64, 0, st>>>(ds, Cds, (int)Nds, tdk, fdk, thr, wnlimit, ranges);
-    k_kadane_apply<<<nblk(Cds * fdk, 8), 256, 0, st>>>(x, ldx, N, Cds * fdk, fdk, ranges);
+    launch_chained(k_kadane_scan, nblk(Cds, 32), 64, 0, st, ds, Cds, (int)Nds, tdk, fdk, thr, wnlimit, ranges);
+    launch_chained(k_kadane_apply, nblk(Cds * fdk, 8), 256, 0, st, x, ldx, N, Cds * fdk, fdk, ranges);
 }
 
 void launch_kadaneT(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
@@ -1433,9 +1453,9 @@ void launch_kadaneT(float *x, long ldx, int C, long N, int tdk, int fdk, float t
     const long Nds = N / tdk;
     if (Cds <= 0 || Nds <= 0) return;
     if (!have_ds) kadane_ds(x, ldx, Cds, Nds, C, N, tdk, fdk, ds, st);
-    k_kadaneT_scan<<<nblk(Nds, 64), 64, 0, st>>>(ds, Cds, Nds, tdk, fdk, thr, bwlimit, ranges);
+    launch_chained(k_kadaneT_scan, nblk(Nds, 64), 64, 0, st, ds, Cds, Nds, tdk, fdk, thr, bwlimit, ranges);
     dim3 g3(nblk(N, 256), Cds * fdk);
-    k_kadaneT_apply<<<g3, 256, 0, st>>>(x, ldx, N, tdk, Nds, ranges);
+    launch_chained(k_kadaneT_apply, g3, 256, 0, st, x, ldx, N, tdk, Nds, ranges);
 }
 
 void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr, float *ds,
@@ -1451,24 +1471,24 @@ void launch_mask(float *x, long ldx, int C, long N, int tdk, int fdk, float thr,
     /* ranks of the quartiles, as the channel zap takes them: sorted[n/4], sorted[n-1-n/4] */
     const uint32_t k0 = (uint32_t)(n / 4), k1 = (uint32_t)(n - 1 - n / 4);
     const unsigned hb = (unsigned)std::min<long>(nblk(n, 256), 152L * 8);
-    for (int shift = 24; shift >= 0; shift -= 8) k_mask_hist<<<hb, 256, 0, st>>>(ds, n, sel, shift, k0, k1, thr);
+    for (int shift = 24; shift >= 0; shift -= 8) launch_chained(k_mask_hist, hb, 256, 0, st, ds, n, sel, shift, k0, k1, thr);
     dim3 g3(nblk(N, 256), Cds * fdk);
-    k_mask_apply<<<g3, 256, 0, st>>>(x, ldx, N, Cds, Nds, tdk, fdk, ds, sel, nzap);
+    launch_chained(k_mask_apply, g3, 256, 0, st, x, ldx, N, Cds, Nds, tdk, fdk, ds, sel, nzap);
 }
 
 void launch_zdot(float *x, long ldx, int C, long N, float *s, double *sstats, float2 *zp,
                  cudaStream_t st)
 {
-    k_zdot_norm<<<C, RB_THREADS, 0, st>>>(x, ldx, N, zp);
-    k_colmean<true><<<nblk(N, 32), dim3(32, CSUM_BLK), 0, st>>>(x, ldx, C, N, nullptr, zp, s);
-    k_zdot_sstats<<<1, 1024, 0, st>>>(s, N, sstats);
+    launch_chained(k_zdot_norm, C, RB_THREADS, 0, st, x, ldx, N, zp);
+    launch_chained(k_colmean<true>, nblk(N, 32), dim3(32, CSUM_BLK), 0, st, x, ldx, C, N, nullptr, zp, s);
+    launch_chained(k_zdot_sstats, 1, 1024, 0, st, s, N, sstats);
     if (N <= ZF_CACHE) {
         const size_t smem = (size_t)(N + 3) / 4 * 16;
         /* per call: the attribute belongs to the current device */
         cudaFuncSetAttribute(k_zdot_fit<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ZF_CACHE * sizeof(float)));
-        k_zdot_fit<true><<<C, RB_THREADS, smem, st>>>(x, ldx, N, zp, s, sstats);
+        launch_chained(k_zdot_fit<true>, C, RB_THREADS, smem, st, x, ldx, N, zp, s, sstats);
     } else {
-        k_zdot_fit<false><<<C, RB_THREADS, 0, st>>>(x, ldx, N, zp, s, sstats);
+        launch_chained(k_zdot_fit<false>, C, RB_THREADS, 0, st, x, ldx, N, zp, s, sstats);
     }
 }
 

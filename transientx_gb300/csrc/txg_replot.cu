@@ -163,6 +163,7 @@ __device__ __forceinline__ void rp_scan(RpTile *tile, const float *rows, long pi
 __global__ void __launch_bounds__(RP_THREADS) k_rp_zdot_sums(const float *__restrict__ buf, const RpMeta *__restrict__ m,
                                                              double *__restrict__ mean, double *__restrict__ std)
 {
+    chain_wait();
     __shared__ RpTile tile[RNB];
     __shared__ double mean_sh[32];
     const RpMeta c = m[blockIdx.y];
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(RP_THREADS) k_rp_zdot_sums(const float *__rest
 __global__ void __launch_bounds__(256) k_rp_zdot_norm(float *__restrict__ buf, const RpMeta *__restrict__ m,
                                                       const double *__restrict__ mean, const double *__restrict__ std)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= c.nchan) return;
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(256) k_rp_zdot_norm(float *__restrict__ buf, c
 __global__ void k_rp_zdot_s(const float *__restrict__ buf, const RpMeta *__restrict__ m,
                             double *__restrict__ s, long soff_stride)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nbin) return;
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(RP_THREADS) k_rp_zdot_fit(const float *__restr
                                                             double *__restrict__ xe_all, double *__restrict__ xs_all,
                                                             double2 *__restrict__ ses)
 {
+    chain_wait();
     __shared__ RpTile tile[RNB];
     __shared__ RpTileD prod[2];
     const RpMeta c = m[blockIdx.y];
@@ -270,6 +274,7 @@ __global__ void __launch_bounds__(256) k_rp_zdot_sub(float *__restrict__ buf, co
                                                      const double *__restrict__ xs_all,
                                                      const double2 *__restrict__ ses)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= c.nchan) return;
@@ -294,6 +299,7 @@ __global__ void __launch_bounds__(RP_THREADS) k_rp_stats(const float *__restrict
                                                          float *__restrict__ skew, float *__restrict__ kurt,
                                                          float *__restrict__ ac)
 {
+    chain_wait();
     __shared__ RpTile tile[2 * RNB];
     __shared__ int first[32];
     __shared__ float shape[32];
@@ -376,6 +382,7 @@ __global__ void __launch_bounds__(256) k_rp_dedisp(const float *__restrict__ src
                                                    const RpMeta *__restrict__ m, const int *__restrict__ delay,
                                                    const long *__restrict__ keep)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= c.nchan) return;
@@ -387,6 +394,7 @@ __global__ void __launch_bounds__(256) k_rp_dedisp(const float *__restrict__ src
 __global__ void __launch_bounds__(256) k_rp_scale(float *__restrict__ buf, const RpMeta *__restrict__ m,
                                                   const float *__restrict__ w)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= c.nchan) return;
@@ -400,6 +408,7 @@ __global__ void __launch_bounds__(256) k_rp_normalize(float *__restrict__ buf, c
                                                       const double *__restrict__ mean,
                                                       const double *__restrict__ var)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= c.nchan) return;
@@ -413,6 +422,7 @@ __global__ void __launch_bounds__(256) k_rp_normalize(float *__restrict__ buf, c
 __global__ void k_rp_clip(float *__restrict__ buf, const RpMeta *__restrict__ m, int td, int fd,
                           float thre)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const long nsds = c.nbin / td, ncds = c.nchan / fd;
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -431,6 +441,7 @@ __global__ void k_rp_clip(float *__restrict__ buf, const RpMeta *__restrict__ m,
 __global__ void __launch_bounds__(128) k_rp_kadane_ds(const float *__restrict__ buf, const RpMeta *__restrict__ m,
                                                       int td, int fd, float *__restrict__ ds, long dstride)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const long nsds = c.nbin / td, ncds = c.nchan / fd;
     const long j = blockIdx.x;
@@ -452,6 +463,7 @@ __global__ void __launch_bounds__(RP_THREADS) k_rp_kadane_scan(const float *__re
                                                                const RpMeta *__restrict__ m, int td, int fd,
                                                                float threshold, long dstride, long *__restrict__ ranges)
 {
+    chain_wait();
     __shared__ RpTile tile[RNB];
     const RpMeta c = m[blockIdx.y];
     const long nsds = c.nbin / td, ncds = c.nchan / fd;
@@ -490,6 +502,7 @@ __global__ void __launch_bounds__(RP_THREADS) k_rp_kadane_scan(const float *__re
 __global__ void __launch_bounds__(128) k_rp_kadane_apply(float *__restrict__ buf, const RpMeta *__restrict__ m, int fd,
                                                          const long *__restrict__ ranges)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= c.nchan / fd * fd) return;
@@ -504,6 +517,7 @@ __global__ void __launch_bounds__(128) k_rp_kadane_apply(float *__restrict__ buf
 __global__ void k_rp_fsum(const float *__restrict__ src, float *__restrict__ dst,
                           const RpMeta *__restrict__ m, int fd)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y]; /* geometry before the downsample */
     const long nc = c.nchan / fd;
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -527,6 +541,7 @@ __global__ void __launch_bounds__(256) k_rp_hough_level(const float *__restrict_
                                                         const int *__restrict__ hrange,
                                                         const int *__restrict__ flip, int t)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const long ncol = c.nbin, r = blockIdx.x;
     if (r >= c.nchans) return;
@@ -558,6 +573,7 @@ __global__ void __launch_bounds__(256) k_rp_hough_level(const float *__restrict_
 __global__ void k_rp_profile(const float *__restrict__ buf, float *__restrict__ h,
                              const RpMeta *__restrict__ m)
 {
+    chain_wait();
     const RpMeta c = m[blockIdx.y];
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nbin) return;
@@ -584,6 +600,7 @@ __global__ void __launch_bounds__(RP_THREADS) k_rp_csum(const float *__restrict_
                                                         const int *__restrict__ rows, double *__restrict__ var_all,
                                                         float *__restrict__ csump)
 {
+    chain_wait();
     __shared__ RpTile tile[RNB];
     __shared__ RpTileD diff[2];
     __shared__ RpTile outt[2];
@@ -642,6 +659,7 @@ __global__ void __launch_bounds__(256) k_rp_match(const RpMeta *__restrict__ m, 
                                                   const float *__restrict__ csump, float *__restrict__ snr,
                                                   int *__restrict__ wid, RpBest *__restrict__ rbest)
 {
+    chain_wait();
     __shared__ float temp[RP_W];
     __shared__ int wns[RP_W];
     __shared__ RpBest red[8];
@@ -704,6 +722,7 @@ __global__ void __launch_bounds__(256) k_rp_match(const RpMeta *__restrict__ m, 
 __global__ void __launch_bounds__(256) k_rp_best(const RpMeta *__restrict__ m, const int *__restrict__ rows,
                                                  const RpBest *__restrict__ rbest, RpBest *__restrict__ best)
 {
+    chain_wait();
     __shared__ RpBest red[256];
     const RpMeta c = m[blockIdx.x];
     RpBest mine{0x7fffffffffffffffL, -1.f, 0};
@@ -893,17 +912,20 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(mem.alloc(&xe, tchan));
         RP_TRY(mem.alloc(&xs, tchan));
         RP_TRY(mem.alloc(&ses, n));
-        k_rp_zdot_sums<<<dim3(per32(maxchan()), NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, mean, var);
-        k_rp_zdot_norm<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
-        k_rp_zdot_s<<<dim3(nblk(maxnbin, 64), NB), 64, 0, st>>>(buf[cur], dmeta, zs, maxnbin);
-        k_rp_zdot_fit<<<dim3(per32(maxchan()) + 1, NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
-        k_rp_zdot_sub<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, zs, maxnbin, xe, xs, ses);
+        launch_chained(k_rp_zdot_sums, dim3(per32(maxchan()), NB), RP_THREADS, 0, st, buf[cur], dmeta, mean, var);
+        launch_chained(k_rp_zdot_norm, dim3(maxchan(), NB), 256, 0, st, buf[cur], dmeta, mean, var);
+        launch_chained(k_rp_zdot_s, dim3(nblk(maxnbin, 64), NB), 64, 0, st, buf[cur], dmeta, zs, maxnbin);
+        launch_chained(k_rp_zdot_fit, dim3(per32(maxchan()) + 1, NB), RP_THREADS, 0, st, buf[cur], dmeta, zs, maxnbin,
+                       xe, xs, ses);
+        launch_chained(k_rp_zdot_sub, dim3(maxchan(), NB), 256, 0, st, buf[cur], dmeta, zs, maxnbin,
+                       xe, xs, ses);
         RP_TRY(cudaGetLastError());
     }
     /* 2: get_stats (their skewness, kurtosis, autocorrelation drive azap) */
     std::vector<float> sk_h(tchan), ku_h(tchan), ac_h(tchan);
     if (upto >= 2) {
-        k_rp_stats<true><<<dim3(per32(maxchan()), NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
+        launch_chained(k_rp_stats<true>, dim3(per32(maxchan()), NB), RP_THREADS, 0, st, buf[cur], dmeta,
+                       mean, var, skew, kurt, ac);
         RP_TRY(cudaGetLastError());
         RP_TRY(cudaMemcpyAsync(sk_h.data(), skew, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
         RP_TRY(cudaMemcpyAsync(ku_h.data(), kurt, sizeof(float) * tchan, cudaMemcpyDeviceToHost, st));
@@ -942,7 +964,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         long *dcut;
         RP_TRY(mem.alloc(&dcut, n));
         RP_TRY(cudaMemcpyAsync(dcut, cut.data(), sizeof(long) * n, cudaMemcpyHostToDevice, st));
-        k_rp_dedisp<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], buf[cur ^ 1], dmeta, delay, dcut);
+        launch_chained(k_rp_dedisp, dim3(maxchan(), NB), 256, 0, st, buf[cur], buf[cur ^ 1], dmeta, delay, dcut);
         RP_TRY(cudaGetLastError());
         RP_TRY(cudaStreamSynchronize(st)); /* dl goes out of scope */
         cur ^= 1;
@@ -969,7 +991,7 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             }
         }
         RP_TRY(cudaMemcpyAsync(w, w_h.data(), sizeof(float) * tchan, cudaMemcpyHostToDevice, st));
-        k_rp_scale<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, w);
+        launch_chained(k_rp_scale, dim3(maxchan(), NB), 256, 0, st, buf[cur], dmeta, w);
         RP_TRY(cudaGetLastError());
     }
     /* 6: zap(zaplist): weights keep azap's zeros */
@@ -980,20 +1002,21 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
                 for (int z = 0; z < o->nzap; z++)
                     if (h.f[j] >= o->zap[z][0] && h.f[j] <= o->zap[z][1]) w_h[h.coff + j] = 0;
         RP_TRY(cudaMemcpyAsync(w, w_h.data(), sizeof(float) * tchan, cudaMemcpyHostToDevice, st));
-        k_rp_scale<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, w);
+        launch_chained(k_rp_scale, dim3(maxchan(), NB), 256, 0, st, buf[cur], dmeta, w);
         RP_TRY(cudaGetLastError());
     }
     /* 7, 8: get_stats, normalize */
     if (upto >= 7)
-        k_rp_stats<false><<<dim3(per32(maxchan()), NB), RP_THREADS, 0, st>>>(buf[cur], dmeta, mean, var, skew, kurt, ac);
+        launch_chained(k_rp_stats<false>, dim3(per32(maxchan()), NB), RP_THREADS, 0, st, buf[cur], dmeta,
+                       mean, var, skew, kurt, ac);
     if (upto >= 8)
-        k_rp_normalize<<<dim3(maxchan(), NB), 256, 0, st>>>(buf[cur], dmeta, mean, var);
+        launch_chained(k_rp_normalize, dim3(maxchan(), NB), 256, 0, st, buf[cur], dmeta, mean, var);
     RP_TRY(cudaGetLastError());
     /* 9: clip */
     if (upto >= 9 && clp) {
         const int td = o->clip[0], fd = o->clip[1];
         const float thre = (float)((float)o->clip[2] * std::sqrt(td * fd));
-        k_rp_clip<<<dim3(nblk(maxelem(), 256), NB), 256, 0, st>>>(buf[cur], dmeta, td, fd, thre);
+        launch_chained(k_rp_clip, dim3(nblk(maxelem(), 256), NB), 256, 0, st, buf[cur], dmeta, td, fd, thre);
         RP_TRY(cudaGetLastError());
     }
     /* 10: kadaneF (nwidth 0, as replot_fil calls it) */
@@ -1009,16 +1032,16 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
             long *rng;
             RP_TRY(mem.alloc(&ds, (size_t)tchan * dstride));
             RP_TRY(mem.alloc(&rng, (size_t)tchan * 4));
-            k_rp_kadane_ds<<<dim3(ncmax, NB), 128, 0, st>>>(buf[cur], dmeta, td, fd, ds, dstride);
-            k_rp_kadane_scan<<<dim3(per32((int)ncmax), NB), RP_THREADS, 0, st>>>(ds, dmeta, td, fd,
+            launch_chained(k_rp_kadane_ds, dim3(ncmax, NB), 128, 0, st, buf[cur], dmeta, td, fd, ds, dstride);
+            launch_chained(k_rp_kadane_scan, dim3(per32((int)ncmax), NB), RP_THREADS, 0, st, ds, dmeta, td, fd,
                                                                                  (float)o->kadane[2], dstride, rng);
-            k_rp_kadane_apply<<<dim3(maxchan(), NB), 128, 0, st>>>(buf[cur], dmeta, fd, rng);
+            launch_chained(k_rp_kadane_apply, dim3(maxchan(), NB), 128, 0, st, buf[cur], dmeta, fd, rng);
             RP_TRY(cudaGetLastError());
         }
     }
     /* 11: downsample(1, fd) */
     if (upto >= 11 && o->fd > 1) {
-        k_rp_fsum<<<dim3(nblk(maxelem(), 256), NB), 256, 0, st>>>(buf[cur], buf[cur ^ 1], dmeta, o->fd);
+        launch_chained(k_rp_fsum, dim3(nblk(maxelem(), 256), NB), 256, 0, st, buf[cur], buf[cur ^ 1], dmeta, o->fd);
         RP_TRY(cudaGetLastError());
         cur ^= 1;
         for (auto &h : H) {
@@ -1111,12 +1134,12 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         const int maxrows = *std::max_element(rows_h.begin(), rows_h.end());
         if (!o->nopt) {
             for (int t = 0; t < maxlevels; t++) {
-                k_rp_hough_level<<<dim3(maxrows, NB), 256, 0, st>>>(buf[cur], hb[hc], hb[hc ^ 1], dmeta, dshift, dhr,
+                launch_chained(k_rp_hough_level, dim3(maxrows, NB), 256, 0, st, buf[cur], hb[hc], hb[hc ^ 1], dmeta, dshift, dhr,
                                                                    dflip, t);
                 hc ^= 1;
             }
         } else {
-            k_rp_profile<<<dim3(nblk(maxnbin, 128), NB), 128, 0, st>>>(buf[cur], hb[0], dmeta);
+            launch_chained(k_rp_profile, dim3(nblk(maxnbin, 128), NB), 128, 0, st, buf[cur], hb[0], dmeta);
         }
         RP_TRY(cudaGetLastError());
         /* boxcar width ladder of matched_filter / peak_search (:979-993), a float vector */
@@ -1150,10 +1173,10 @@ extern "C" int txg_replot(const txg_replot_opts *o, const txg_replot_cand *cands
         RP_TRY(mem.alloc(&dvar, nrows));
         RP_TRY(mem.alloc(&drbest, nrows));
         RP_TRY(mem.alloc(&dbest, n));
-        k_rp_csum<<<dim3(per32(maxrows), NB), RP_THREADS, 0, st>>>(hb[hc], dmeta, drows, dvar, csump);
-        k_rp_match<<<dim3(maxrows, NB), 256, 0, st>>>(dmeta, drows, dvwn, dnbox, wstride, dvar, csump, dsnr, dwidm,
+        launch_chained(k_rp_csum, dim3(per32(maxrows), NB), RP_THREADS, 0, st, hb[hc], dmeta, drows, dvar, csump);
+        launch_chained(k_rp_match, dim3(maxrows, NB), 256, 0, st, dmeta, drows, dvwn, dnbox, wstride, dvar, csump, dsnr, dwidm,
                                                      drbest);
-        k_rp_best<<<NB, 256, 0, st>>>(dmeta, drows, drbest, dbest);
+        launch_chained(k_rp_best, NB, 256, 0, st, dmeta, drows, drbest, dbest);
         RP_TRY(cudaGetLastError());
         RP_TRY(cudaMemcpyAsync(best.data(), dbest, sizeof(RpBest) * n, cudaMemcpyDeviceToHost, st));
         RP_TRY(cudaStreamSynchronize(st));
