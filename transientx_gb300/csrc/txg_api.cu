@@ -569,7 +569,6 @@ int run_block(txg_handle *h, int beam, const uint8_t *raw, const float *rawf = n
         int rc = harvest(h, b, sl, P);
         if (rc && rc != TXG_ERR_OVERFLOW) return rc;
         if (rc) status = rc;
-        TXG_CUDA_TRY(cudaStreamWaitEvent(rs, h->fork, 0));
         if (timing) TXG_CUDA_TRY(cudaEventRecord(sl.ev[0], rs));
 
         TXG_CUDA_TRY(cudaMemsetAsync(sl.dcount, 0, 2 * sizeof(int), rs));
@@ -581,6 +580,9 @@ int run_block(txg_handle *h, int beam, const uint8_t *raw, const float *rawf = n
             TXG_CUDA_TRY(cudaMemcpy2DAsync(xcur, P.ldh * sizeof(float), xprev + P.N,
                                            P.ldh * sizeof(float), P.H * sizeof(float), P.C,
                                            cudaMemcpyDeviceToDevice, rs));
+        /* what came so far is the row's own and runs beside the channel zap; the block's samples and
+         * mask are the handle stream's */
+        TXG_CUDA_TRY(cudaStreamWaitEvent(rs, h->fork, 0));
         float *x = xcur + P.H;
         bool part = false;
         if (rawf)

