@@ -140,7 +140,7 @@ def class_bytes(info, sp, nchans_raw, ndump_raw, ncand, elem):
             series + 4.0 * info.ndm * info.nsamples, 4.0 * info.ndm * info.nsamples + 16 * ncand]
 
 
-RFI_LAUNCHES = {"kadaneF": 3, "kadaneT": 3, "zdot": 4, "zero": 2, "mask": 10}
+RFI_LAUNCHES = {"kadaneF": 3, "kadaneT": 3, "zdot": 4, "zero": 2, "mask": 6}
 BOXCAR_ROW_MAX = 51200  # samples of a dedispersed row one boxcar CTA holds; longer rows: 2 kernels
 
 
@@ -152,8 +152,8 @@ S1_SETS, S1_GPT = 16, 4  # default stage-1 shapes: 16 thread sets of 4 coarse-DM
 
 
 def stage1_window_loads(d1):
-    """Window elements stage 1 loads per output sample, summed over channels and thread sets,
-    at the default launch shapes: a thread set loads a channel's window values for its first
+    """Window elements stage 1 loads per output sample (from tensor memory by default, from shared
+    memory in the other shapes), summed over channels and thread sets: a thread set loads a channel's window values for its first
     group and again wherever the delay differs from the previous group's (groups past the end
     repeat the last delay)."""
     ng, C = d1.shape
@@ -164,11 +164,12 @@ def stage1_window_loads(d1):
 
 
 def class_smem_bytes(info, elem, d1):
-    """Shared-memory bytes one launch of the classes bound by shared memory loads: stage 1 one
+    """On-chip bytes one launch of the dedispersion and boxcar classes loads: stage 1 one
     FP32 window element per sample for each delay change within a thread set's groups (the
-    loads the kernel makes; additions are C x ngroup x N), stage 2 one ring element (elem
+    loads the kernel makes, from tensor memory by default; additions are C x ngroup x N), stage 2 one ring element (elem
     bytes) per addition (nsub x ndm x (N + noverlap)), the boxcar two running-sum values per
-    (sample, width).  Other classes: None."""
+    (sample, width) of a search over every width, of which it skips what its bounds allow.  Other
+    classes: None."""
     return [None, None, 4.0 * info.ndump * stage1_window_loads(d1),
             float(elem) * info.nsub * info.ndm * info.nsamples,
             8.0 * info.ndm * info.nsamples * info.nwidths]

@@ -347,8 +347,9 @@ int txg_get_timing(txg_handle *h, double *ms, int64_t *launches, int32_t n);
 /* txg_get_timing for one ddplan row (its own accumulators, reset by this call). */
 int txg_get_row_timing(txg_handle *h, int32_t row, double *ms, int64_t *launches, int32_t n);
 
-/* The dedispersion launch shapes a row runs with: stage1 = resident stage-1 shape (time tile
- * x coarse-DM groups per CTA), stage2 = stage-2 threads-per-CTA variant, stage2_kb = its
+/* The dedispersion launch shapes a row runs with: stage1 = stage-1 shape (0 = from tensor memory, 18
+ * where that does not apply; others a time tile x coarse-DM groups per CTA), stage2 = stage-2
+ * threads-per-CTA variant (3 to 5: at most 8 DMs a CTA), stage2_kb = its
  * shared-memory budget in KB (0 = default); see txg_dedisp.cu.  With TXG_FLAG_AUTOTUNE they
  * are the fastest of a few candidates timed at txg_create (all candidates give bit-identical
  * results; the subband count and DM group stay as planned, since they change the sums).  No

@@ -1,5 +1,9 @@
 """Copies by several threads and scratch memory that calls share: large blocks whose size is no
 multiple of a part, and calls of different sizes from several threads at once."""
+import ctypes
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -8,10 +12,28 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("ndump,nchans", [(2048, 512), (2050, 1023), (4097, 1025), (8191, 1024)])
+def _child(*what):
+    """In a process of its own: what is allocated in these threads and freed by this one would
+    otherwise serve the tests after it."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), *what], cwd=root, capture_output=True, text=True,
+                       timeout=300, env={**os.environ, "PYTHONPATH": root})
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 @pytest.mark.parametrize("kind", ["u8", "f32"])
-def test_pageable_blocks_arrive_as_pinned_ones(tx, ndump, nchans, kind):
-    torch = pytest.importorskip("torch")
+@pytest.mark.parametrize("size", ["2048x512", "2050x1023", "4097x1025", "8191x1024"])
+def test_pageable_blocks_arrive_as_pinned_ones(size, kind):
+    _child(size, kind)
+
+
+def test_calls_share_scratch_between_threads():
+    _child("threads")
+
+
+def _blocks(ndump, nchans, kind):
+    import transientx_gb300 as tx
+    rt = ctypes.CDLL("libcudart.so")
     rng = np.random.default_rng(ndump)
     blocks = [rng.integers(90, 160, (ndump, nchans)).astype(np.uint8) for _ in range(4)]
     if kind == "f32":
@@ -23,10 +45,16 @@ def test_pageable_blocks_arrive_as_pinned_ones(tx, ndump, nchans, kind):
         with tx.Search([row], nchans, 256e-6, f, ndump, flags=tx.FLAG_KEEP_SERIES, zapthre=0.0) as s:
             got = []
             for b in blocks:
+                p = ctypes.c_void_p()
                 if pinned:
-                    b = torch.from_numpy(b).pin_memory().numpy()
+                    assert rt.cudaHostAlloc(ctypes.byref(p), ctypes.c_size_t(b.nbytes), 0) == 0
+                    q = np.frombuffer((ctypes.c_char * b.nbytes).from_address(p.value), b.dtype).reshape(b.shape)
+                    q[:] = b
+                    b = q
                 (s.push_block if kind == "u8" else s.push_block_f32)(b)
                 s.sync()
+                if pinned:
+                    assert rt.cudaFreeHost(p) == 0
                 if s.row_info(0).gated:
                     got.append(s.timdata(0).copy())
         out.append(got)
@@ -35,7 +63,8 @@ def test_pageable_blocks_arrive_as_pinned_ones(tx, ndump, nchans, kind):
         np.testing.assert_array_equal(a, b)
 
 
-def test_calls_share_scratch_between_threads(tx):
+def _calls_from_threads():
+    import transientx_gb300 as tx
     rng = np.random.default_rng(5)
     widths = tx.width_ladder(1e-4, 0.05, 0.1, 1e-4)
     sizes = [(3, 70), (40, 9001), (256, 8192), (90, 62496), (1500, 1024)]
@@ -64,3 +93,10 @@ def test_calls_share_scratch_between_threads(tx):
     for t in threads:
         t.join()
     assert not bad, bad[0]
+
+
+if __name__ == "__main__":
+    if sys.argv[1] == "threads":
+        _calls_from_threads()
+    else:
+        _blocks(*map(int, sys.argv[1].split("x")), sys.argv[2])

@@ -9,8 +9,10 @@
  * Stage 2: for fine DM k of group g and output sample i of the gated block
  *     tim[k][i] = sum_{s ascending} sub[g][s][t0 + i + d2[k][s]].
  *
- * Both kernels stage their input windows in shared memory with the Blackwell bulk-copy
- * engine (cp.async.bulk global->shared, completion tracked by an mbarrier with a bounded
+ * By default stage 1 copies a subband's channel windows to shared memory with cp.async and from
+ * there, as lanes of sixteen samples, to tensor memory, from which the sums are read at any column
+ * (k_stage1t).  Its other shapes and stage 2 stage their input windows in shared memory with the
+ * bulk-copy engine (cp.async.bulk global->shared, completion tracked by an mbarrier with a bounded
  * wait): one window per channel row (stage 1) or per subband ring segment (stage 2), so each
  * input element crosses HBM/L2 once per CTA tile.  A wait that runs out sets *err and the
  * CTA returns without touching its outputs.
