@@ -1,5 +1,5 @@
-"""The dedispersion kernels that sum from tensor memory against the shared-memory ones over plans
-at their edges: the same additions in the same order, so the series are equal bit for bit."""
+"""Stage 1 from tensor memory, and stage 2 as it is by default, against the shared-memory shapes over
+plans at their edges: the same additions in the same order, so the series are equal bit for bit."""
 import numpy as np
 import pytest
 
